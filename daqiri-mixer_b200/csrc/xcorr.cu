@@ -25,16 +25,28 @@
 // 128 x 128-byte boxes)
 // into a 3-deep shared-memory ring.  One elected thread issues all
 // tcgen05.mma; the int32 accumulators stay in TMEM for the whole K range of
-// the launch; eight epilogue warps read them back with tcgen05.ld and add
-// them into the tile-packed int32 or int64 cube in HBM.
+// the launch; eight epilogue warps read them back with tcgen05.ld into
+// registers, release TMEM and add them into the tile-packed int32 or int64
+// cube in HBM while the next tile's MMAs run.
 //
-// Warp roles (320 threads with the default build, one CTA per SM, persistent
-// over work items):
+// What bounds it: the int8 tensor rate at the clock the 1000 W cap leaves for
+// long K, the cube's read-modify-write in HBM for short K.  One tile's four
+// products fill TMEM, so the next tile waits for the drain alone (about 1 us)
+// instead of for the adds: 128 result registers a thread, which the register
+// split below pays for.  One B200, against adds straight from TMEM: 4096
+// elements x 64 channels, K 2048 with its corner-turn 5.81 -> 5.49 ms; 1024 x
+// 64, K 2048 int64 328 -> 301 us, K 8192 802 -> 782 us; 200 x 128, K 1536
+// int32 and flush 121 -> 117 us; 48 small arrays in one launch 573 -> 557 us;
+// 1024 elements, K 1024 and K 32 768: the same within 0.4 %.
+//
+// Warp roles (384 threads, one CTA per SM, persistent over work items):
 //   warp 0      TMA producer; picks the CTA's next item and passes its index
 //               to the other roles through a shared-memory ring
 //   warp 1      TMEM allocator + MMA issuer
-//   warps 2..9  epilogue (TMEM lane quadrant = warp % 4, 64-column half =
-//               (warp - 2) / 4)
+//   warps 2, 3  idle (they complete the first warpgroup, whose registers go
+//               to the epilogue)
+//   warps 4..11 epilogue (TMEM lane quadrant = warp % 4, every other
+//               16-column chunk)
 // A single-array launch hands CTA b the items b, b + grid, ... (all items
 // but the ragged block's cost the same); a table launch takes items in list
 // order from a global counter, so CTAs stay on neighbouring items, which
@@ -49,32 +61,12 @@ namespace mixer {
 namespace {
 
 // Pipeline geometry (build-time options): samples per stage (128 with the
-// 128-byte swizzle or 64 with the 64-byte swizzle), stage count, and epilogue
-// warps per TMEM lane quadrant.
+// 128-byte swizzle or 64 with the 64-byte swizzle) and stage count.
 #ifndef MIXER_XCORR_KC
 #define MIXER_XCORR_KC 128
 #endif
 #ifndef MIXER_XCORR_STAGES
 #define MIXER_XCORR_STAGES 3
-#endif
-#ifndef MIXER_XCORR_EPI_GROUPS
-#define MIXER_XCORR_EPI_GROUPS 2
-#endif
-// int64 epilogue of an item that owns its tile: 1 = load, add, store; 0 = the
-// 64-bit atomic add (fire and forget) that K-split items always use.  Measured
-// on B200 the load-add-store form is 5 % faster at K 1024 per launch but 21 %
-// slower at 256 elements and K 256 (its loads wait on DRAM latency), so the
-// atomic add is the default.
-#ifndef MIXER_XCORR_EXCL_RMW
-#define MIXER_XCORR_EXCL_RMW 0
-#endif
-// Diagonal tiles (i == j) with three products instead of four: there
-// P1 = Xi Xr^T = P2^T, so one M 128 x N 256 MMA gives [R1 | P2], one
-// M 128 x N 128 MMA gives R2 = Xi Xi^T, and the epilogue forms
-// Im = P2^T - P2 by exchanging 32 x 32 blocks of P2 through shared memory.
-// 0: four products on every tile.
-#ifndef MIXER_XCORR_DIAG3
-#define MIXER_XCORR_DIAG3 0
 #endif
 // Tiles of a ragged last block (N not a multiple of 128) with the block on the
 // MMA's N side, N = 2 r16 (1), or as full 128 x 128 tiles with zero rows (0).
@@ -95,10 +87,13 @@ constexpr int kStages = MIXER_XCORR_STAGES;
 constexpr int kTileBytes = kTile * kKc;
 constexpr int kStageBytes = 4 * kTileBytes;      // Ar, Ai, Br, Bi
 static_assert(kKc == 64 || kKc == 128, "stage of 64 or 128 samples");
-constexpr int kEpiGroups = MIXER_XCORR_EPI_GROUPS;  // column groups per TMEM lane quadrant
+constexpr int kEpiGroups = 2;                    // epilogue warps per TMEM lane quadrant
 constexpr int kEpiWarps = 4 * kEpiGroups;
 constexpr int kEpiCols = kTile / kEpiGroups;     // 64 columns per warp
-constexpr int kThreads = 64 + 32 * kEpiWarps;
+constexpr int kEpiChunks = kEpiCols / 16;        // 16-column chunks per warp
+constexpr int kEpiWarp0 = 4;                     // first epilogue warp
+constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
+constexpr int kPairThreads = 64 + 32 * kEpiWarps;
 constexpr int kBarBytes = 512;
 // Item ring (table launches take items from a global counter): the producer
 // publishes each item index to the MMA and epilogue warps through kItemSlots
@@ -107,28 +102,16 @@ constexpr int kItemSlots = 8;
 constexpr int kItemBar0 = 24;                    // first ring barrier (uint64 index)
 static_assert(2 * MIXER_XCORR_STAGES + 5 <= kItemBar0, "barrier area");
 static_assert((kItemBar0 + 3 * kItemSlots) * 8 <= kBarBytes, "barrier area");
-// The diagonal-tile exchange needs the 2 x 4 layout of eight epilogue warps.
-constexpr bool kDiag3 = MIXER_XCORR_DIAG3 != 0 && kEpiGroups == 2;
-// Exchange area: one round's eight 32 x 32 int32 blocks of P2, rows padded to
-// 33 words so that both the row-wise writes and the column-wise reads of a
-// warp hit 32 different banks.
-constexpr int kXchgStride = 33;
-constexpr int kXchgBlock = 32 * kXchgStride;     // words per block
-constexpr int kXchgBytes = kDiag3 ? 8 * kXchgBlock * 4 : 0;
 // Transpose area of the ragged tiles: per epilogue warp 32 rows of 16 words,
 // padded to 17 (row writes and the two-rows-per-read pattern are conflict-free).
-// It shares the exchange area (the two serve different items).
 constexpr int kXposeStride = 17;
 constexpr int kXposeBytes =
     (MIXER_XCORR_TAIL && MIXER_XCORR_TAIL_XPOSE) ? kEpiWarps * 32 * kXposeStride * 4 : 0;
-constexpr int kEpiSmemBytes = kXchgBytes > kXposeBytes ? kXchgBytes : kXposeBytes;
 constexpr int kSmemBase = kStages * kStageBytes + 1024 + kBarBytes;
-constexpr int kSmemBytes = kSmemBase + kEpiSmemBytes;   // the most a launch asks for
+constexpr int kSmemBytes = kSmemBase + kXposeBytes;   // the most a launch asks for
 static_assert(kSmemBytes <= 232448, "shared memory");
 constexpr uint32_t kTmemCols = 512;              // D1 (256) + D2 (256)
 constexpr uint32_t kIdesc = idesc_i8(128, 256);
-constexpr uint32_t kIdescN128 = idesc_i8(128, 128);
-constexpr int kEpiBarrier = 1;                   // named barrier of the eight epilogue warps
 
 struct XcorrArgs {
     int32_t nant, nch, nblk, ntiles;
@@ -245,21 +228,18 @@ __device__ __forceinline__ void tmem_ld4_x16(uint32_t a0, uint32_t a1, uint32_t 
         : "memory");
 }
 
-// One and three 32x32b.x16 TMEM loads (16 columns each) with their wait.
-__device__ __forceinline__ void tmem_ld_x16(uint32_t a, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(a)
-        : "memory");
+// Register split: the launch gives 384 threads 168 registers each; the four
+// control warps keep kCtrlRegs and the eight epilogue warps take kEpiRegs,
+// which hold a warp's whole share of a tile (128 values a thread).
+constexpr int kCtrlRegs = 56, kEpiRegs = 224;
+static_assert(4 * kCtrlRegs + 8 * kEpiRegs <= 12 * 168, "register split");
+template <int R>
+__device__ __forceinline__ void reg_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
 }
-
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+template <int R>
+__device__ __forceinline__ void reg_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
 }
 
 // Adds (or stores) 16 elements of one row of TMEM into the cube: element e at
@@ -269,22 +249,7 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
 template <int kStride>
 __device__ __forceinline__ void store16(const Item& it, size_t e0, const int32_t (&re)[16],
                                         const int32_t (&im)[16]) {
-    if (it.mode == MIXER_VIS_ACC_I64 && MIXER_XCORR_EXCL_RMW && it.excl) {
-        // the item owns the tile: a warp reads, adds and writes 256 contiguous
-        // bytes per column and plane
-        long long* v = reinterpret_cast<long long*>(it.vis) + e0;
-        long long a[16], b[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            a[e] = v[e * kStride];
-            b[e] = v[e * kStride + kTile * kTile];
-        }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            v[e * kStride] = a[e] + (long long)re[e];
-            v[e * kStride + kTile * kTile] = b[e] + (long long)im[e];
-        }
-    } else if (it.mode == MIXER_VIS_ACC_I64) {
+    if (it.mode == MIXER_VIS_ACC_I64) {
         unsigned long long* v = reinterpret_cast<unsigned long long*>(it.vis) + e0;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -310,10 +275,7 @@ __device__ __forceinline__ void store16(const Item& it, size_t e0, const int32_t
 
 // Adds (or stores) one element of the cube, in the item's mode.
 __device__ __forceinline__ void store1(const Item& it, size_t e, int32_t x) {
-    if (it.mode == MIXER_VIS_ACC_I64 && MIXER_XCORR_EXCL_RMW && it.excl) {
-        long long* v = reinterpret_cast<long long*>(it.vis) + e;
-        *v += (long long)x;
-    } else if (it.mode == MIXER_VIS_ACC_I64) {
+    if (it.mode == MIXER_VIS_ACC_I64) {
         atomicAdd(reinterpret_cast<unsigned long long*>(it.vis) + e, (unsigned long long)(long long)x);
     } else if (it.mode == MIXER_VIS_ACC_I32) {
         atomicAdd(reinterpret_cast<int*>(it.vis) + e, x);
@@ -369,6 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    if (warp < kEpiWarp0) reg_dec<kCtrlRegs>();
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         if (lane == 0) {
@@ -476,16 +439,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // 256-row B operand [Xr_j ; Xi_j]: two adjacent tiles (2 it.tail
                     // rows for a ragged block)
                     const uint64_t b = (diag && !it.tail) ? ar : sdesc(sb + 2 * kTileBytes);
-                    // diagonal tiles: D2 = Xi Xi^T (N 128) instead of Xi [Xr ; Xi]^T
-                    const bool three = kDiag3 && diag && !it.tail;
-                    const uint64_t b2 = three ? ai : b;
-                    const uint32_t id2 = three ? kIdescN128 : id1;
 #pragma unroll
                     for (int kk = 0; kk < kKc / 32; ++kk) {
                         const uint64_t o = (uint64_t)((kk * 32) >> 4);   // 32-byte K step
                         const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
                         mma_i8(t_d1, ar + o, b + o, id1, acc);
-                        mma_i8(t_d2, ai + o, b2 + o, id2, acc);
+                        mma_i8(t_d2, ai + o, b + o, id1, acc);
                     }
                     tc_commit(bar(EMPTY + stage));   // stage free once these MMAs finish
                     if (++stage == kStages) {
@@ -505,15 +464,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_commit(bar(DRAIN));
             mbar_wait(bar(DRAIN), 0);
         }
-    } else {
+    } else if (warp >= kEpiWarp0) {
         // ------------------------------------------------------------ epilogue
-        // Eight warps: TMEM lane quadrant warp % 4, column half (warp - 2) / 4.
-        // Each warp reads its 64 columns 16 at a time and adds them into the
-        // cube; TMEM is released once every warp has read its last chunk.
+        // Eight warps: TMEM lane quadrant warp % 4, every other 16-column chunk.
+        // Each warp reads its (up to 64) columns of the four products into 128
+        // registers, releases TMEM to the next tile's MMAs and then adds.
+        reg_inc<kEpiRegs>();
         const int q = warp & 3;
-        const int col0 = kEpiCols * ((warp - 2) >> 2);
+        const int g = (warp - kEpiWarp0) >> 2;
         const int m = q * 32 + lane;
-        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)col0;
+        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
         uint32_t acc_phase = 0;
         int islot = 0;
         uint32_t iphase = 0;
@@ -539,146 +499,71 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc_fence_after();
             const size_t tb = ((size_t)it.c * it.ntiles + it.t) * (size_t)(2 * kTile * kTile);
-            if (it.tail) {
-                // Ragged last block on the N side: columns n < it.tail of each
-                // product (R1 | P2 at 0 | it.tail, P1 | R2 at 256 | 256 + it.tail).
-                // Transposed tile (i != j): TMEM row m is column m of tile (i, j)
-                // and column n its row n, so Re = R1 + R2, Im = P2 - P1 and the
-                // 16 values of a load belong to 16 consecutive rows.  Chunks of
-                // 16 columns alternate between the column groups; in store mode
-                // the rows past it.tail are written as zeros.
-                const bool tr = it.i != it.j;
-                const int g = (warp - 2) >> 2;
-                const int nt = it.tail;
-                const int ncols = it.mode == MIXER_VIS_STORE_I32 ? kTile : nt;
-                const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
-                int last = -1;   // this warp's last chunk that reads TMEM
-                for (int n0 = 16 * g; n0 < nt; n0 += 16 * kEpiGroups) last = n0;
-                if (last < 0) {
-                    tc_fence_before();
-                    mbar_arrive(bar(ACCE));
-                }
-#pragma unroll 1
-                for (int n0 = 16 * g; n0 < ncols; n0 += 16 * kEpiGroups) {
-                    int32_t re[16], im[16];
-                    if (n0 < nt) {
-                        uint32_t r[4][16];   // R1, P2, P1, R2
-                        tmem_ld4_x16(tq + n0, tq + nt + n0, tq + 256 + n0, tq + 256 + nt + n0, r);
-                        if (n0 == last) {
-                            tc_fence_before();
-                            mbar_arrive(bar(ACCE));
-                        }
+            // Columns n < nt of each product: R1 | P2 at 0 | nt, P1 | R2 at
+            // 256 | 256 + nt; nt = 128 or, for the ragged last block on the N
+            // side, its rows.  Transposed tile (ragged, i != j): TMEM row m is
+            // column m of tile (i, j) and column n its row n, so Re = R1 + R2,
+            // Im = P2 - P1.  Columns past nt are zeros (store mode writes them).
+            const bool tr = it.tail && it.i != it.j;
+            const int nt = it.tail ? it.tail : kTile;
+            int32_t re[kEpiChunks][16], im[kEpiChunks][16];
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            re[e] = (int32_t)(r[0][e] + r[3][e]);
-                            im[e] = tr ? (int32_t)(r[1][e] - r[2][e]) : (int32_t)(r[2][e] - r[1][e]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) re[e] = im[e] = 0;
-                    }
-                    if (tr && it.mode == MIXER_VIS_STORE_I32 &&
-                        (reinterpret_cast<uintptr_t>(it.vis) & 15) == 0) {
-                        // stores: a thread's 16 elements are contiguous, 4 x 16 bytes
-                        int4* vr = reinterpret_cast<int4*>(reinterpret_cast<int*>(it.vis) + tb +
-                                                           (size_t)m * kTile + n0);
-                        int4* vi = vr + kTile * kTile / 4;
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            vr[e] = make_int4(re[4 * e], re[4 * e + 1], re[4 * e + 2], re[4 * e + 3]);
-                            vi[e] = make_int4(im[4 * e], im[4 * e + 1], im[4 * e + 2], im[4 * e + 3]);
-                        }
-                    } else if (tr && kXposeBytes) {
-                        // row `lane` of the warp's 32 x 16 block -> pairs of rows,
-                        // 16 consecutive elements each, per instruction
-                        int32_t* xs = xchg + (warp - 2) * 32 * kXposeStride;
-                        const int rr = lane >> 4, cc = lane & 15;
-#pragma unroll 1
-                        for (int pl = 0; pl < 2; ++pl) {
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) xs[lane * kXposeStride + e] = pl ? im[e] : re[e];
-                            __syncwarp();
-                            const size_t pb = tb + (size_t)pl * kTile * kTile + n0 + cc;
-#pragma unroll 4
-                            for (int s2 = 0; s2 < 16; ++s2) {
-                                const int row = 2 * s2 + rr;
-                                store1(it, pb + (size_t)(q * 32 + row) * kTile,
-                                       xs[row * kXposeStride + cc]);
-                            }
-                            __syncwarp();
-                        }
-                    } else if (tr) {
-                        store16<1>(it, tb + (size_t)m * kTile + n0, re, im);
-                    } else {
-                        store16<kTile>(it, tb + (size_t)n0 * kTile + m, re, im);
-                    }
-                }
-            } else if (!(kDiag3 && it.i == it.j)) {
-#pragma unroll 1
-                for (int n0 = 0; n0 < kEpiCols; n0 += 16) {
+            for (int k = 0; k < kEpiChunks; ++k) {
+                const int n0 = 16 * (kEpiGroups * k + g);
+                if (n0 < nt) {
                     uint32_t r[4][16];   // R1, P2, P1, R2
-                    tmem_ld4_x16(trow + n0, trow + 128 + n0, trow + 256 + n0, trow + 384 + n0, r);
-                    if (n0 == kEpiCols - 16) {           // this warp's TMEM reads are done
-                        tc_fence_before();
-                        mbar_arrive(bar(ACCE));
-                    }
-                    int32_t re[16], im[16];
+                    tmem_ld4_x16(tq + n0, tq + nt + n0, tq + 256 + n0, tq + 256 + nt + n0, r);
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        re[e] = (int32_t)(r[0][e] + r[3][e]);
-                        im[e] = (int32_t)(r[2][e] - r[1][e]);
+                        re[k][e] = (int32_t)(r[0][e] + r[3][e]);
+                        im[k][e] = tr ? (int32_t)(r[1][e] - r[2][e]) : (int32_t)(r[2][e] - r[1][e]);
                     }
-                    store16<kTile>(it, tb + (size_t)(col0 + n0) * kTile + m, re, im);
-                }
-            } else {
-                // Diagonal tile: TMEM holds R1 (columns 0-127), P2 (128-255) and
-                // R2 (256-383); Im[m][n] = P2[n][m] - P2[m][n].  Warp (q, h) owns
-                // rows 32q.. and columns 64h..; it needs P2[n][m] for n in its
-                // columns, i.e. the 32 x 32 blocks of P2 at rows of quadrants
-                // 2h, 2h+1 and columns 32q.., which the warps of those quadrants
-                // read from TMEM and pass through shared memory.  Round rho: the
-                // warps of quadrants 2rho, 2rho+1 write their blocks (slot =
-                // (quadrant - 2rho) * 4 + consumer quadrant), then the warps of
-                // column half rho read them transposed and write their rows.
-                const int hq = (warp - 2) >> 2;
-#pragma unroll 1
-                for (int rho = 0; rho < 2; ++rho) {
-                    if ((q >> 1) == rho) {
-#pragma unroll 1
-                        for (int g = 0; g < 4; ++g) {
-                            uint32_t p[16];
-                            tmem_ld_x16(trow + 128 + 16 * g, p);
-                            const int qc = 2 * hq + (g >> 1);
-                            int32_t* dst = xchg + ((q - 2 * rho) * 4 + qc) * kXchgBlock +
-                                           lane * kXchgStride + 16 * (g & 1);
+                } else {
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) dst[e] = (int32_t)p[e];
-                        }
-                    }
-                    named_bar_sync(kEpiBarrier, 32 * kEpiWarps);
-                    if (hq == rho) {
-#pragma unroll 1
-                        for (int n0 = 0; n0 < kEpiCols; n0 += 16) {
-                            uint32_t r1[16], p2[16], r2[16];
-                            tmem_ld_x16(trow + n0, r1);
-                            tmem_ld_x16(trow + 128 + n0, p2);
-                            tmem_ld_x16(trow + 256 + n0, r2);
-                            int32_t re[16], im[16];
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) {
-                                const int ep = n0 + e;     // column within this warp's 64
-                                const int32_t p2t = xchg[((ep >> 5) * 4 + q) * kXchgBlock +
-                                                         (ep & 31) * kXchgStride + lane];
-                                re[e] = (int32_t)(r1[e] + r2[e]);
-                                im[e] = (int32_t)((uint32_t)p2t - p2[e]);
-                            }
-                            store16<kTile>(it, tb + (size_t)(col0 + n0) * kTile + m, re, im);
-                        }
-                    }
-                    named_bar_sync(kEpiBarrier, 32 * kEpiWarps);   // blocks consumed
+                    for (int e = 0; e < 16; ++e) re[k][e] = im[k][e] = 0;
                 }
-                tc_fence_before();
-                mbar_arrive(bar(ACCE));                 // every TMEM read of the tile done
+            }
+            tc_fence_before();
+            mbar_arrive(bar(ACCE));                  // TMEM is free for the next tile
+            const int ncols = it.mode == MIXER_VIS_STORE_I32 ? kTile : nt;
+#pragma unroll
+            for (int k = 0; k < kEpiChunks; ++k) {
+                const int n0 = 16 * (kEpiGroups * k + g);
+                if (n0 >= ncols) break;
+                if (!tr) {
+                    store16<kTile>(it, tb + (size_t)n0 * kTile + m, re[k], im[k]);
+                } else if (it.mode == MIXER_VIS_STORE_I32 &&
+                           (reinterpret_cast<uintptr_t>(it.vis) & 15) == 0) {
+                    // stores: a thread's 16 elements are contiguous, 4 x 16 bytes
+                    int4* vr = reinterpret_cast<int4*>(reinterpret_cast<int*>(it.vis) + tb +
+                                                       (size_t)m * kTile + n0);
+                    int4* vi = vr + kTile * kTile / 4;
+#pragma unroll
+                    for (int e = 0; e < 16; e += 4) {
+                        vr[e / 4] = make_int4(re[k][e], re[k][e + 1], re[k][e + 2], re[k][e + 3]);
+                        vi[e / 4] = make_int4(im[k][e], im[k][e + 1], im[k][e + 2], im[k][e + 3]);
+                    }
+                } else {
+                    // row `lane` of the warp's 32 x 16 block -> pairs of rows,
+                    // 16 consecutive elements each, per instruction
+                    int32_t* xs = xchg + (warp - kEpiWarp0) * 32 * kXposeStride;
+                    const int rr = lane >> 4, cc = lane & 15;
+#pragma unroll
+                    for (int pl = 0; pl < 2; ++pl) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            xs[lane * kXposeStride + e] = pl ? im[k][e] : re[k][e];
+                        __syncwarp();
+                        const size_t pb = tb + (size_t)pl * kTile * kTile + n0 + cc;
+#pragma unroll 4
+                        for (int s2 = 0; s2 < 16; ++s2) {
+                            const int row = 2 * s2 + rr;
+                            store1(it, pb + (size_t)(q * 32 + row) * kTile,
+                                   xs[row * kXposeStride + cc]);
+                        }
+                        __syncwarp();
+                    }
+                }
             }
             acc_phase ^= 1u;
         }
@@ -771,7 +656,7 @@ __device__ __forceinline__ PairHalf pair_half(const PairArgs& g, int64_t w, int 
     return h;
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kPairThreads, 1)
     k_xcorr_pair(const __grid_constant__ CUtensorMap tmap, const PairArgs args) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -1092,7 +977,6 @@ int xcorr_encode_maps(CUtensorMap* maps, const int8_t* planes, int32_t nant, int
 // ragged-block tiles (measured: the larger carve-out slows the int64
 // epilogue of other launches by up to 5 %).
 static int launch_smem(bool ragged) {
-    if (kDiag3) return kSmemBytes;
     return kSmemBase + ((MIXER_XCORR_TAIL && ragged) ? kXposeBytes : 0);
 }
 
@@ -1128,7 +1012,7 @@ static int pair_clusters() {
             at[0].val.clusterDim.y = 1;
             at[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3(2 * 74);
-            cfg.blockDim = dim3(kThreads);
+            cfg.blockDim = dim3(kPairThreads);
             cfg.dynamicSmemBytes = kPairSmemBytes;
             cfg.attrs = at;
             cfg.numAttrs = 1;
@@ -1179,7 +1063,7 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(2 * ncl));
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = kPairSmemBytes;
     cfg.stream = st;
     cfg.attrs = at;
