@@ -45,9 +45,7 @@ struct mixer_batch {
     int64_t nwork;
     int32_t split[kMaxClass + 1];
     int32_t order;
-    int32_t grid;
     int32_t* d_err;
-    unsigned long long* d_ctr;   // item counter of the launch
     bool ragged;                 // some array's N is not a multiple of 128
     cudaGraph_t graph;
     cudaGraphExec_t exec;
@@ -126,7 +124,6 @@ extern "C" int mixer_batch_destroy(mixer_batch* b) {
     cudaFree(b->d_probs);
     cudaFree(b->d_work);
     cudaFree(b->d_err);
-    cudaFree(b->d_ctr);
     delete b;
     return MIXER_OK;
 }
@@ -185,14 +182,12 @@ extern "C" int mixer_batch_create(const mixer_xcorr_problem* probs, int32_t npro
     if ((e = cudaMalloc(&b->d_maps, maps.size() * sizeof(CUtensorMap))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_probs, nprob * sizeof(mixer::XcorrProblem))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_err, sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_ctr, sizeof(unsigned long long))) != cudaSuccess ||
         (e = cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap),
                         cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(b->d_probs, b->tprobs.data(), nprob * sizeof(mixer::XcorrProblem),
                         cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemset(b->d_err, 0, sizeof(int32_t))) != cudaSuccess)
         return fail(mixer::cuda_status(e, "batch tables"));
-    b->grid = mixer::xcorr_sm_count();
     rc = upload_plan(b);
     if (rc != MIXER_OK) return fail(rc);
     *out = b;
@@ -212,9 +207,8 @@ extern "C" int mixer_batch_plan(mixer_batch* b, const int32_t* split_per_class, 
 
 extern "C" int mixer_batch_run(mixer_batch* b, void* stream) {
     if (!b) return MIXER_EINVAL;
-    return mixer::xcorr_launch_table(b->d_maps, b->d_probs, b->d_work, b->nwork, b->grid, b->d_err,
-                                     b->d_ctr, b->ragged,
-                                     static_cast<cudaStream_t>(stream));
+    return mixer::xcorr_launch_table(b->d_maps, b->d_probs, b->d_work, b->nwork, b->d_err,
+                                     b->ragged, static_cast<cudaStream_t>(stream));
 }
 
 static int time_plan(mixer_batch* b, int reps, cudaStream_t st, float* ms) {

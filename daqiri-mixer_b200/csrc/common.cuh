@@ -97,6 +97,35 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// ---- dynamic work: cluster launch control -----------------------------------
+// A running CTA takes over ("cancels") a CTA of its own launch that has not
+// started yet: the 16-byte answer lands in shared memory and completes 16
+// bytes on an mbarrier.  No further request may follow one that found none.
+__device__ __forceinline__ void clc_request(uint32_t dst, uint32_t bar) {
+    asm volatile(
+        "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128"
+        " [%0], [%1];" ::"r"(dst),
+        "r"(bar)
+        : "memory");
+}
+// blockIdx.x of the CTA taken over, or -1 when every CTA has started.  The
+// fence orders this read before the next request's write to the same bytes.
+__device__ __forceinline__ int64_t clc_answer(uint32_t src) {
+    uint32_t x, ok;
+    asm volatile(
+        "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+        "ld.shared.b128 h, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+        "selp.u32 %1, 1, 0, p;\n\t"
+        "mov.u32 %0, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t"
+        "fence.proxy.async.shared::cta;\n\t}"
+        : "=r"(x), "=r"(ok)
+        : "r"(src)
+        : "memory");
+    return ok ? (int64_t)x : -1;
+}
+
 // ---- tcgen05 ------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),

@@ -168,7 +168,6 @@ struct mixer_server {
     bool table_used[2] = {false, false};
     int tsel = 0;
     int32_t* d_err = nullptr;
-    unsigned long long* d_ctr = nullptr;   // item counter of the GEMM launches (stream comp)
     // Stream state comes from a server-owned stream-ordered pool and pinned dump
     // buffers are recycled, so opening or closing a stream never runs the
     // device-wide synchronisation of cudaMalloc / cudaFree / cudaFreeHost while
@@ -346,8 +345,7 @@ bool serve_once(mixer_server* sv) {
     cudaMemcpyAsync(sv->d_work[ts], sv->h_work[ts], work.size() * sizeof(mixer::XcorrWork),
                     cudaMemcpyHostToDevice, comp);
     const int rc = mixer::xcorr_launch_table(sv->d_maps[ts], sv->d_probs[ts], sv->d_work[ts],
-                                             (int64_t)work.size(), mixer::xcorr_sm_count(), sv->d_err,
-                                             sv->d_ctr, ragged, comp);
+                                             (int64_t)work.size(), sv->d_err, ragged, comp);
     if (rc != MIXER_OK) sv->error.store(rc);
     cudaEventRecord(sv->table_free[ts], comp);
     sv->table_used[ts] = true;
@@ -540,8 +538,7 @@ extern "C" int mixer_server_create(const mixer_server_cfg* cfg, mixer_server** o
             return fail(e, "server tables");
     }
     if ((e = cudaMalloc(&sv->d_err, sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMemset(sv->d_err, 0, sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMalloc(&sv->d_ctr, sizeof(unsigned long long))) != cudaSuccess)
+        (e = cudaMemset(sv->d_err, 0, sizeof(int32_t))) != cudaSuccess)
         return fail(e, "server error word");
     sv->worker = std::thread(worker_main, sv);
     *out = sv;
@@ -575,7 +572,6 @@ extern "C" int mixer_server_destroy(mixer_server* sv) {
         if (sv->table_free[t]) cudaEventDestroy(sv->table_free[t]);
     }
     cudaFree(sv->d_err);
-    cudaFree(sv->d_ctr);
     if (sv->copy) cudaStreamDestroy(sv->copy);
     if (sv->comp) cudaStreamDestroy(sv->comp);
     if (sv->d2h) cudaStreamDestroy(sv->d2h);

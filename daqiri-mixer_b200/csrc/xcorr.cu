@@ -47,10 +47,11 @@
 //               to the epilogue)
 //   warps 4..11 epilogue (TMEM lane quadrant = warp % 4, every other
 //               16-column chunk)
-// A single-array launch hands CTA b the items b, b + grid, ... (all items
-// but the ragged block's cost the same); a table launch takes items in list
-// order from a global counter, so CTAs stay on neighbouring items, which
-// share operand blocks in L2, whatever each item costs.
+// The grid is one CTA per item, of which one per SM runs at a time; the
+// running CTAs take over the waiting ones' items in list order (cluster launch
+// control), so they stay on neighbouring items, which share operand blocks in
+// L2, whatever each item costs.  Launches with few items per SM, and those
+// with a CTA limit, hand CTA b the items b, b + grid, ... (launch_grid).
 #include "common.cuh"
 #include "xcorr.cuh"
 #include <cstdlib>
@@ -95,13 +96,13 @@ constexpr int kEpiWarp0 = 4;                     // first epilogue warp
 constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 constexpr int kPairThreads = 64 + 32 * kEpiWarps;
 constexpr int kBarBytes = 512;
-// Item ring (table launches take items from a global counter): the producer
-// publishes each item index to the MMA and epilogue warps through kItemSlots
-// slots after the pipeline barriers.
+// Item ring: the producer publishes each item index to the MMA and epilogue
+// warps through kItemSlots slots after the pipeline barriers.
 constexpr int kItemSlots = 8;
 constexpr int kItemBar0 = 24;                    // first ring barrier (uint64 index)
 static_assert(2 * MIXER_XCORR_STAGES + 5 <= kItemBar0, "barrier area");
-static_assert((kItemBar0 + 3 * kItemSlots) * 8 <= kBarBytes, "barrier area");
+constexpr int kClcSlot = (kItemBar0 + 3 * kItemSlots) * 8;   // 16-byte launch-control answer
+static_assert(kClcSlot % 16 == 0 && kClcSlot + 16 <= kBarBytes, "barrier area");
 // Transpose area of the ragged tiles: per epilogue warp 32 rows of 16 words,
 // padded to 17 (row writes and the two-rows-per-read pattern are conflict-free).
 constexpr int kXposeStride = 17;
@@ -117,13 +118,11 @@ struct XcorrArgs {
     int32_t nant, nch, nblk, ntiles;
     int32_t kbeg, nkc;   // first sample, number of 128-sample chunks
     int32_t mode;
-    int32_t pad_;
+    int32_t dynamic;     // 1: one CTA per item, taken over by the running ones; 0: CTA b
+                         // takes items b, b + grid, ...
     int64_t nwork;       // nch * ntiles, or the length of `work`
     void* vis;
     int32_t* err;
-    // Item counter of a table launch, zero at its start (nullptr: CTA b takes
-    // items b, b + grid, ...).
-    unsigned long long* ctr;
     // Batched mode (work != nullptr): per-array tensor maps, problems, work list.
     // Two maps per array: [2p] the 128-row operand boxes, [2p + 1] the ragged
     // last block's box over both planes.
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int FULL = 0, EMPTY = kStages, ACCF = 2 * kStages, ACCE = 2 * kStages + 1,
-              DRAIN = 2 * kStages + 2, IFULL = kItemBar0, IEMPTY = kItemBar0 + kItemSlots;
+              DRAIN = 2 * kStages + 2, CLC = 2 * kStages + 3, IFULL = kItemBar0, IEMPTY = kItemBar0 + kItemSlots;
     auto bar = [&](int k) { return smem_u32(&bars[k]); };
 
     if (threadIdx.x == 0) {
@@ -311,6 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         mbar_init(bar(ACCF), 1);
         mbar_init(bar(ACCE), 32 * kEpiWarps);
         mbar_init(bar(DRAIN), 1);
+        mbar_init(bar(CLC), 1);
         for (int s = 0; s < kItemSlots; ++s) {
             mbar_init(bar(IFULL + s), 1);
             mbar_init(bar(IEMPTY + s), 1 + kEpiWarps);   // the MMA thread, one per epilogue warp
@@ -342,6 +342,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             int islot = 0;
             uint32_t iphase = 0;
             int64_t w = blockIdx.x;
+            uint32_t clc_phase = 0;
+            bool asked = false;   // a request for the next item is under way
+            const uint32_t clc_slot = smem_u32(gbase + kStages * kStageBytes + kClcSlot);
             while (ok) {
                 // publish the item (or the end mark -1) to the MMA and epilogue warps
                 if (w >= args.nwork) w = -1;
@@ -356,6 +359,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     iphase ^= 1u;
                 }
                 if (w < 0) break;
+                if (args.dynamic) {
+                    // ask for the next item now: the answer comes during this one
+                    mbar_expect_tx(bar(CLC), 16);
+                    clc_request(clc_slot, bar(CLC));
+                    asked = true;
+                }
                 const Item it = get_item(args, &tmap, &tmap_tail, w);
                 const bool diag = (it.i == it.j);
                 const uint32_t bytes = it.tail ? 2 * kTileBytes + 2 * it.tail * kKc
@@ -386,9 +395,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                         phase ^= 1u;
                     }
                 }
-                // next item: in list order from the launch's counter, or round robin
-                w = args.ctr ? (int64_t)gridDim.x + (int64_t)atomicAdd(args.ctr, 1ull)
-                             : w + gridDim.x;
+                if (!args.dynamic) {
+                    w += gridDim.x;
+                } else if (ok && mbar_wait(bar(CLC), clc_phase, abort_flag)) {
+                    clc_phase ^= 1u;
+                    asked = false;
+                    w = clc_answer(clc_slot);
+                } else {
+                    ok = false;
+                }
             }
             if (!ok) {
                 if (args.err) atomicOr(args.err, 1);
@@ -396,6 +411,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // Let the copies already issued land before the CTA exits.
                 for (int64_t q = issued - 1; q >= 0 && q >= issued - kStages; --q)
                     mbar_wait(bar(FULL + (int)(q % kStages)), (uint32_t)((q / kStages) & 1));
+                // Take over the CTAs that have not started, so that the launch
+                // ends here instead of giving each of them its own time-out.
+                while (args.dynamic && w >= 0) {
+                    if (!asked) {
+                        mbar_expect_tx(bar(CLC), 16);
+                        clc_request(clc_slot, bar(CLC));
+                    }
+                    asked = false;
+                    if (!mbar_wait(bar(CLC), clc_phase)) break;
+                    clc_phase ^= 1u;
+                    w = clc_answer(clc_slot);
+                }
             }
         }
     } else if (warp == 1) {
@@ -1072,6 +1099,24 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
     return MIXER_OK;
 }
 
+// Grid of a launch, and how its CTAs find their items.  Round robin leaves the
+// SMs that reach their memory more slowly behind: at 1024 elements, K 1024,
+// where the cube's read-modify-write is the bound, the SMs were busy for 82 %
+// of the launch.  Taken over one by one the items even that out.  One B200,
+// round robin -> taken over, int64: 1024 x 64, K 1024 256 -> 238 us; 4096 x 8,
+// K 1024 457 -> 410 us; 640 x 48 (4.9 items an SM) the same.  Below four items
+// an SM there is little to even out, and which SMs get the last round's items
+// matters more: 256 x 128 (2.6 an SM), K 1024 55 -> 57 us, so those stay round
+// robin.  Table launches hold items of different lengths and are always taken
+// over; a launch with a CTA limit cannot be, since its grid would be the items.
+static int64_t launch_grid(XcorrArgs& a, int32_t max_ctas) {
+    const int64_t sms = sm_count();
+    a.dynamic = max_ctas <= 0 && a.nwork <= INT32_MAX && a.nwork > (a.work ? sms : 4 * sms);
+    if (a.dynamic) return a.nwork;
+    const int64_t grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+    return a.nwork < grid ? a.nwork : grid;
+}
+
 // Launch over samples [kbeg, kbeg + klen) with klen <= MIXER_KMAX_I32.
 // At most max_ctas persistent CTAs (<= 0: one per SM).
 static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t kt, int64_t kbeg,
@@ -1095,17 +1140,13 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
     a.kbeg = (int32_t)kbeg;
     a.nkc = (int32_t)((klen + kWorkChunk - 1) / kWorkChunk);
     a.mode = mode;
-    a.pad_ = 0;
     a.nwork = (int64_t)nch * a.ntiles;
     a.vis = vis;
     a.err = err;
-    a.ctr = nullptr;
     a.tmaps = nullptr;
     a.probs = nullptr;
     a.work = nullptr;
-    int64_t grid = sm_count();
-    if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
-    if (a.nwork < grid) grid = a.nwork;
+    const int64_t grid = launch_grid(a, max_ctas);
     k_xcorr_tri<<<(unsigned)grid, kThreads, launch_smem(nant % kTile != 0), st>>>(maps[0], maps[1],
                                                                                   a);
     MIXER_CK(cudaGetLastError());
@@ -1113,24 +1154,22 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
 }
 
 int xcorr_launch_table(const CUtensorMap* d_tmaps, const XcorrProblem* d_probs,
-                       const XcorrWork* d_work, int64_t nwork, int grid, int32_t* err,
-                       unsigned long long* ctr, bool ragged, cudaStream_t st) {
-    if (nwork <= 0 || grid <= 0 || !ctr) return MIXER_EINVAL;
+                       const XcorrWork* d_work, int64_t nwork, int32_t* err, bool ragged,
+                       cudaStream_t st) {
+    if (nwork <= 0) return MIXER_EINVAL;
     int rc = set_smem_attr();
     if (rc != MIXER_OK) return rc;
-    MIXER_CK(cudaMemsetAsync(ctr, 0, sizeof(*ctr), st));
     XcorrArgs a;
     memset(&a, 0, sizeof(a));
     a.nwork = nwork;
     a.err = err;
-    a.ctr = ctr;
     a.tmaps = d_tmaps;
     a.probs = d_probs;
     a.work = d_work;
     CUtensorMap unused;
     memset(&unused, 0, sizeof(unused));
-    k_xcorr_tri<<<(unsigned)(grid < nwork ? grid : nwork), kThreads, launch_smem(ragged), st>>>(
-        unused, unused, a);
+    k_xcorr_tri<<<(unsigned)launch_grid(a, 0), kThreads, launch_smem(ragged), st>>>(unused, unused,
+                                                                                    a);
     MIXER_CK(cudaGetLastError());
     return MIXER_OK;
 }

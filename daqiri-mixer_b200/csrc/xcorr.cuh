@@ -30,13 +30,12 @@ int xcorr_encode_map(CUtensorMap* map, const int8_t* planes, int32_t nant, int32
 // ragged last 128-row block (both planes in one box).
 int xcorr_encode_maps(CUtensorMap* maps, const int8_t* planes, int32_t nant, int32_t nch, int64_t kt,
                       int64_t kend);
-// One persistent launch over a device work list (`grid` CTAs at most; d_tmaps
-// holds two maps per array, from xcorr_encode_maps).  The CTAs take items in
-// list order from *ctr (device memory of the caller's, zeroed on `st` before
-// the launch); ragged: some array's N is not a multiple of 128.
+// One persistent launch over a device work list, whose items the CTAs take in
+// list order (d_tmaps holds two maps per array, from xcorr_encode_maps);
+// ragged: some array's N is not a multiple of 128.
 int xcorr_launch_table(const CUtensorMap* d_tmaps, const XcorrProblem* d_probs,
-                       const XcorrWork* d_work, int64_t nwork, int grid, int32_t* err,
-                       unsigned long long* ctr, bool ragged, cudaStream_t st);
+                       const XcorrWork* d_work, int64_t nwork, int32_t* err, bool ragged,
+                       cudaStream_t st);
 int xcorr_sm_count();
 
 }  // namespace mixer

@@ -543,3 +543,29 @@ def test_image_matches_reference_publish_path(cuda):
         got = img.cpu().numpy().reshape(128, 32, 32)
     scale = np.abs(ref_img).max(axis=(1, 2), keepdims=True)
     assert np.all(np.abs(got - ref_img) <= 1e-4 * scale)
+
+
+# ------------------------------------------- items taken over while a launch runs
+
+@pytest.mark.parametrize("nant,nch,klen", [
+    (24, 592, 96),       # 4 items per SM: the last round-robin launch
+    (24, 593, 96),       # the first whose CTAs take over the waiting ones' items
+    (24, 2000, 256),     # many rounds of short items
+    (130, 198, 144),     # ragged tiles among them
+])
+def test_xcorr_items_taken_over(cuda, nant, nch, klen):
+    import torch
+    rng = np.random.default_rng(nch)
+    planes = _rand_planes(rng, nch, nant, klen)
+    ref = oracle.vis_tile_pack(oracle.correlate(planes)).reshape(-1)
+    dpl = _t(planes, cuda)
+    err = _zeros(1, torch.int32, cuda)
+    for mode, dtype, times in ((mixer.VIS_STORE_I32, torch.int32, 1),
+                               (mixer.VIS_ACC_I32, torch.int32, 2),
+                               (mixer.VIS_ACC_I64, torch.int64, 2)):
+        vis = _zeros(ref.size, dtype, cuda)
+        for _ in range(2):
+            mixer.xcorr_tri(dpl, nant, nch, klen, 0, klen, mode, vis, err)
+        _sync()
+        assert np.array_equal(vis.cpu().numpy().astype(np.int64), times * ref), mode
+    assert int(err.item()) == 0
