@@ -569,3 +569,34 @@ def test_xcorr_items_taken_over(cuda, nant, nch, klen):
         _sync()
         assert np.array_equal(vis.cpu().numpy().astype(np.int64), times * ref), mode
     assert int(err.item()) == 0
+
+
+# ------------------------------------- corner-turn groups that do not divide evenly
+
+@pytest.mark.parametrize("nant,nch,tpkt,nheaps,k0", [
+    (3, 5, 16, 1, 0),        # one heap
+    (5, 7, 32, 9, 16),       # last group of one heap
+    (4, 127, 32, 15, 0),     # last groups of heaps and of channels both short
+    (6, 43, 48, 7, 48),      # rows of 12 vectors: the block is no multiple of them
+    (2, 3, 4112, 2, 0),      # rows wider than the block (257 vectors)
+    (700, 16, 16, 3, 0),     # more CTAs than a short grid
+])
+def test_corner_turn_remainders(cuda, nant, nch, tpkt, nheaps, k0):
+    import torch
+    rng = np.random.default_rng(nant)
+    stride = 64 + 2 * nch * tpkt
+    pk = rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)
+    kt = (k0 + nheaps * tpkt + 16 + 15) // 16 * 16
+    planes = torch.full((2, nch, nant, kt), 7, dtype=torch.int8, device=cuda)
+    dpk = _t(pk, cuda)
+    seq_err = _zeros(1, torch.int32, cuda)
+    err = _zeros(1, torch.int32, cuda)
+    mixer.restamp_seq(dpk, nheaps * nant, stride, 11)
+    mixer.corner_turn(dpk, stride, 64, nant, nch, tpkt, nheaps, 11, planes, kt, k0, seq_err, err)
+    mixer.corner_turn(dpk, stride, 64, nant, nch, tpkt, nheaps, 12, planes, kt, k0, seq_err, err)
+    _sync()
+    got = planes.cpu().numpy()
+    ref = oracle.corner_turn(pk, nant, nch, tpkt, nheaps)
+    assert np.array_equal(got[:, :, :, k0:k0 + nheaps * tpkt], ref)
+    assert np.all(got[:, :, :, :k0] == 7) and np.all(got[:, :, :, k0 + nheaps * tpkt:] == 7)
+    assert int(seq_err.item()) == nheaps * nant and int(err.item()) == 0
