@@ -7,6 +7,7 @@
 // outputs, and host packets are staged through two device buffers on a copy
 // stream so the next copy overlaps the current corner-turn + GEMM (the
 // reference's NBATCH ring and copy / compute streams, :44-45, :146-172).
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <cstdio>
@@ -33,7 +34,8 @@ struct mixer_ctx {
     int64_t* vis64;
     int32_t* vis32;
     int8_t* planes;
-    int64_t kt_max;
+    int64_t kt_max;      // samples of max_heaps heaps
+    int64_t kt_planes;   // samples the planes hold (at least kt_max)
     uint8_t* stage[2];
     size_t stage_bytes;
     cudaEvent_t stage_free[2];
@@ -133,6 +135,33 @@ extern "C" int mixer_destroy(mixer_ctx* c) {
     return MIXER_OK;
 }
 
+// Planes longer than max_heaps, so that a call with more heaps in device memory
+// contracts them in few launches: every launch reads and writes the whole cube
+// once.  One B200, one launch per 32 heaps -> these lengths: the reference's
+// array, 512 heaps and dump 1368 -> 751 us (787 with 8192 samples, 870 with
+// 4096); 1024 elements x 256 channels, 256 heaps 9.50 -> 4.32 ms; 60 x 64, 300
+// heaps in chunks of 8 615 -> 116 us.  Past 1 GiB of planes the shorter length
+// costs nothing (1024 x 256: 4.32 against 4.33 ms).  At most a sixteenth of
+// the device's free memory goes into it; otherwise, or when the allocation
+// fails, the planes hold max_heaps.
+constexpr int64_t kPlaneSamples = 16384, kPlaneSamplesBig = 8192;
+constexpr int64_t kPlaneBytes = 1LL << 30;
+
+static bool alloc_long_planes(mixer_ctx* c) {
+    const int64_t rows = 2LL * c->d.nch * c->d.nant;
+    const int64_t kt = rows * kPlaneSamples <= kPlaneBytes ? kPlaneSamples : kPlaneSamplesBig;
+    size_t free_b = 0, total_b = 0;
+    if (c->kt_max >= kt || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+        (size_t)(rows * kt) > free_b / 16 ||
+        cudaMalloc(&c->planes, (size_t)(rows * kt)) != cudaSuccess) {
+        cudaGetLastError();
+        c->planes = nullptr;
+        return false;
+    }
+    c->kt_planes = kt;
+    return true;
+}
+
 extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     if (!out) return MIXER_EINVAL;
     *out = nullptr;
@@ -157,7 +186,10 @@ extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     c->kt_max = (c->kt_max + 15) / 16 * 16;
     CK_OR_FREE(cudaMalloc(&c->vis64, (size_t)c->vis_elems * sizeof(int64_t)));
     CK_OR_FREE(cudaMemset(c->vis64, 0, (size_t)c->vis_elems * sizeof(int64_t)));
-    CK_OR_FREE(cudaMalloc(&c->planes, (size_t)2 * d->nch * d->nant * c->kt_max));
+    if (!alloc_long_planes(c)) {
+        c->kt_planes = c->kt_max;
+        CK_OR_FREE(cudaMalloc(&c->planes, (size_t)2 * d->nch * d->nant * c->kt_max));
+    }
     const int G = c->d.grid;
     CK_OR_FREE(cudaMalloc(&c->grid, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
     CK_OR_FREE(cudaMalloc(&c->grid_prev, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
@@ -194,7 +226,9 @@ extern "C" int mixer_reset(mixer_ctx* c, void* stream) {
     return MIXER_OK;
 }
 
-// Corner-turn + GEMM over nheaps heaps, staged in chunks of max_heaps.
+// Corner-turn + GEMM over nheaps heaps: host packets in chunks of max_heaps (the
+// staging buffers; the copy over PCIe hides the launches), device packets in
+// equal chunks of at most the planes' length.
 static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uint32_t seq0,
                           int32_t on_device, void* stream, int32_t mode, void* vis) {
     if (!c || !packets || nheaps <= 0) return MIXER_EINVAL;
@@ -202,8 +236,13 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint8_t* src = static_cast<const uint8_t*>(packets);
     const int64_t heap_bytes = (int64_t)d.nant * d.pkt_stride;
-    for (int64_t h0 = 0; h0 < nheaps; h0 += d.max_heaps) {
-        const int32_t nh = (int32_t)((nheaps - h0) < d.max_heaps ? (nheaps - h0) : d.max_heaps);
+    const int64_t most =
+        on_device ? std::max<int64_t>(c->kt_planes / d.tpkt, d.max_heaps) : d.max_heaps;
+    const int64_t chunks = (nheaps + most - 1) / most;
+    const int64_t step = on_device ? (nheaps + chunks - 1) / chunks : most;
+    const int64_t kt = step > d.max_heaps ? (step * d.tpkt + 127) / 128 * 128 : c->kt_max;
+    for (int64_t h0 = 0; h0 < nheaps; h0 += step) {
+        const int32_t nh = (int32_t)((nheaps - h0) < step ? (nheaps - h0) : step);
         const uint8_t* chunk = src + h0 * heap_bytes;
         const uint8_t* dev_chunk = chunk;
         if (!on_device) {
@@ -218,9 +257,9 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
         }
         const uint32_t sq = seq0 + (uint32_t)(h0 * d.nant);
         int rc = mixer_corner_turn(dev_chunk, d.pkt_stride, d.hdr_bytes, d.nant, d.nch, d.tpkt, nh,
-                                   sq, c->planes, c->kt_max, 0, c->d_seq_err, c->d_err, stream);
+                                   sq, c->planes, kt, 0, c->d_seq_err, c->d_err, stream);
         if (rc != MIXER_OK) return rc;
-        rc = mixer_xcorr_tri(c->planes, d.nant, d.nch, c->kt_max, 0, (int64_t)nh * d.tpkt, mode, vis,
+        rc = mixer_xcorr_tri(c->planes, d.nant, d.nch, kt, 0, (int64_t)nh * d.tpkt, mode, vis,
                              c->d_err, stream);
         if (rc != MIXER_OK) return rc;
         if (!on_device) {

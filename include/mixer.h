@@ -279,7 +279,11 @@ typedef struct mixer_array_desc {
     int32_t grid;        /* image grid side G (0: 2 * max(side_x, side_y))    */
     int32_t pkt_stride;  /* bytes between packets in input buffers            */
     int32_t hdr_bytes;   /* payload offset inside a packet                    */
-    int32_t max_heaps;   /* most heaps per antenna given to one correlate call */
+    int32_t max_heaps;   /* most heaps per antenna given to one correlate call;
+                          * longer calls run in chunks: of max_heaps from host
+                          * memory, of up to 16384 samples from device memory
+                          * where a sixteenth of the free memory holds the
+                          * context's planes of that length                  */
 } mixer_array_desc;
 
 typedef struct mixer_ctx mixer_ctx;

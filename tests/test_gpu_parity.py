@@ -600,3 +600,33 @@ def test_corner_turn_remainders(cuda, nant, nch, tpkt, nheaps, k0):
     assert np.array_equal(got[:, :, :, k0:k0 + nheaps * tpkt], ref)
     assert np.all(got[:, :, :, :k0] == 7) and np.all(got[:, :, :, k0 + nheaps * tpkt:] == 7)
     assert int(seq_err.item()) == nheaps * nant and int(err.item()) == 0
+
+
+# ---------------------------------- context calls longer than max_heaps, in chunks
+
+@pytest.mark.parametrize("nheaps", [2, 3, 1024, 1025])   # the planes hold 1024 heaps of 16
+@pytest.mark.parametrize("on_device", [True, False])
+@pytest.mark.parametrize("i32", [False, True])
+def test_context_long_calls(cuda, nheaps, on_device, i32):
+    import torch
+    nant, nch, tpkt = 5, 3, 16
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(nheaps)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    mixer.restamp_seq(pk, nheaps * nant, stride, 7)
+    _sync()
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    src = pk if on_device else pk.cpu().pin_memory()
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=3, grid=16,
+                            pkt_stride=stride, max_heaps=2) as ctx:
+        if i32:
+            ctx.correlate_i32(src, nheaps, 7, on_device=on_device)
+            ctx.integrate()
+        else:
+            ctx.correlate(src, nheaps, 7, on_device=on_device)
+        out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+        ctx.read_vis_i64(out)
+        _sync()
+        assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
+        st = ctx.stats()
+        assert st["samples"] == nheaps * tpkt and st["seq_errors"] == 0 and st["kernel_err"] == 0
