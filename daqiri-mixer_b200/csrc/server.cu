@@ -296,7 +296,7 @@ bool serve_once(mixer_server* sv) {
         maps.push_back(m[1]);
         // one item per (channel, tile) over all ready sub-integrations, and every
         // stream has a cube of its own: the items own their tiles
-        probs.push_back(mixer::XcorrProblem{s.d.nant, s.d.nch, ntiles, 0, MIXER_VIS_ACC_I64, 1, s.vis});
+        probs.push_back(mixer::XcorrProblem{s.d.nant, s.d.nch, ntiles, 0, MIXER_VIS_ACC_I64, s.vis});
         for (int32_t c = 0; c < s.d.nch; ++c)
             for (int t = 0; t < ntiles; ++t) {
                 mixer::XcorrWork it;

@@ -31,13 +31,15 @@
 //
 // What bounds it: the int8 tensor rate at the clock the 1000 W cap leaves for
 // long K, the cube's read-modify-write in HBM for short K.  One tile's four
-// products fill TMEM, so the next tile waits for the drain alone (about 1 us)
-// instead of for the adds: 128 result registers a thread, which the register
-// split below pays for.  One B200, against adds straight from TMEM: 4096
+// products fill TMEM, so the next tile waits for the drain alone (1350 clocks,
+// and 350 more of barriers) instead of for the adds: 128 result registers a
+// thread, which the register split below pays for.  One B200, against adds straight from TMEM: 4096
 // elements x 64 channels, K 2048 with its corner-turn 5.81 -> 5.49 ms; 1024 x
 // 64, K 2048 int64 328 -> 301 us, K 8192 802 -> 782 us; 200 x 128, K 1536
 // int32 and flush 121 -> 117 us; 48 small arrays in one launch 573 -> 557 us;
-// 1024 elements, K 1024 and K 32 768: the same within 0.4 %.
+// 1024 elements, K 1024 and K 32 768: the same within 0.4 %.  D1 is drained
+// first, and the next tile's first D1 MMAs run while D2 is read: 4096 x 64, K
+// 2048 step another 2 %, int32 at K 1024 3-4 %.
 //
 // Warp roles (384 threads, one CTA per SM, persistent over work items):
 //   warp 0      TMA producer; picks the CTA's next item and passes its index
@@ -69,17 +71,6 @@ namespace {
 #ifndef MIXER_XCORR_STAGES
 #define MIXER_XCORR_STAGES 3
 #endif
-// Tiles of a ragged last block (N not a multiple of 128) with the block on the
-// MMA's N side, N = 2 r16 (1), or as full 128 x 128 tiles with zero rows (0).
-#ifndef MIXER_XCORR_TAIL
-#define MIXER_XCORR_TAIL 1
-#endif
-// Transposed ragged tiles: each warp passes its 32 x 16 blocks through shared
-// memory so that a warp's adds cover two 128-byte lines per instruction (1),
-// or adds straight from the TMEM rows, 32 lines per instruction (0).
-#ifndef MIXER_XCORR_TAIL_XPOSE
-#define MIXER_XCORR_TAIL_XPOSE 1
-#endif
 constexpr int kTile = 128;                       // tile rows = cols
 constexpr int kWorkChunk = 128;                  // samples per work-list K unit
 constexpr int kKc = MIXER_XCORR_KC;              // samples (bytes) per pipeline stage
@@ -100,14 +91,13 @@ constexpr int kBarBytes = 512;
 // warps through kItemSlots slots after the pipeline barriers.
 constexpr int kItemSlots = 8;
 constexpr int kItemBar0 = 24;                    // first ring barrier (uint64 index)
-static_assert(2 * MIXER_XCORR_STAGES + 5 <= kItemBar0, "barrier area");
+static_assert(2 * MIXER_XCORR_STAGES + 6 <= kItemBar0, "barrier area");
 constexpr int kClcSlot = (kItemBar0 + 3 * kItemSlots) * 8;   // 16-byte launch-control answer
 static_assert(kClcSlot % 16 == 0 && kClcSlot + 16 <= kBarBytes, "barrier area");
 // Transpose area of the ragged tiles: per epilogue warp 32 rows of 16 words,
 // padded to 17 (row writes and the two-rows-per-read pattern are conflict-free).
 constexpr int kXposeStride = 17;
-constexpr int kXposeBytes =
-    (MIXER_XCORR_TAIL && MIXER_XCORR_TAIL_XPOSE) ? kEpiWarps * 32 * kXposeStride * 4 : 0;
+constexpr int kXposeBytes = kEpiWarps * 32 * kXposeStride * 4;
 constexpr int kSmemBase = kStages * kStageBytes + 1024 + kBarBytes;
 constexpr int kSmemBytes = kSmemBase + kXposeBytes;   // the most a launch asks for
 static_assert(kSmemBytes <= 232448, "shared memory");
@@ -147,7 +137,7 @@ struct Item {
     const CUtensorMap* map;
     const CUtensorMap* map_tail;
     void* vis;
-    int c, t, i, j, kbeg, kc0, nkc, mode, ntiles, excl;
+    int c, t, i, j, kbeg, kc0, nkc, mode, ntiles;
     int tail;   // rows per plane of the ragged last block on the N side (0: full tile)
 };
 
@@ -173,7 +163,6 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
         it.nkc = a.nkc;
         it.mode = a.mode;
         it.ntiles = a.ntiles;
-        it.excl = 1;          // one launch, one item per (channel, tile)
     } else {
         const XcorrWork wk = a.work[w];
         const XcorrProblem& pr = a.probs[wk.prob];
@@ -188,11 +177,10 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
         it.nkc = (int)wk.nkc;
         it.mode = pr.mode;
         it.ntiles = pr.ntiles;
-        it.excl = pr.excl;
     }
     decode_tile(it.t, it.i, it.j);
     const int r16 = tail_rows(nant);
-    it.tail = (MIXER_XCORR_TAIL && r16 < kTile && it.i == (nant - 1) / kTile) ? r16 : 0;
+    it.tail = (r16 < kTile && it.i == (nant - 1) / kTile) ? r16 : 0;
     return it;
 }
 
@@ -227,10 +215,59 @@ __device__ __forceinline__ void tmem_ld4_x16(uint32_t a0, uint32_t a1, uint32_t 
         : "memory");
 }
 
+// Eight loads of 16 columns (four of D1's first half 32 columns apart, four of
+// its second half) and the wait, likewise in one statement.
+__device__ __forceinline__ void tmem_ld8_x16(uint32_t a, uint32_t b, uint32_t (&p)[64],
+                                             uint32_t (&q)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%128];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%129];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%130];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%131];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%64,%65,%66,%67,%68,%69,%70,%71,%72,%73,%74,%75,%76,%77,%78,%79}, [%132];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95}, [%133];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%96,%97,%98,%99,%100,%101,%102,%103,%104,%105,%106,%107,%108,%109,%110,%111}, [%134];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%112,%113,%114,%115,%116,%117,%118,%119,%120,%121,%122,%123,%124,%125,%126,%127}, [%135];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(p[0]), "=r"(p[1]), "=r"(p[2]), "=r"(p[3]), "=r"(p[4]), "=r"(p[5]), "=r"(p[6]),
+          "=r"(p[7]), "=r"(p[8]), "=r"(p[9]), "=r"(p[10]), "=r"(p[11]), "=r"(p[12]),
+          "=r"(p[13]), "=r"(p[14]), "=r"(p[15]), "=r"(p[16]), "=r"(p[17]), "=r"(p[18]),
+          "=r"(p[19]), "=r"(p[20]), "=r"(p[21]), "=r"(p[22]), "=r"(p[23]), "=r"(p[24]),
+          "=r"(p[25]), "=r"(p[26]), "=r"(p[27]), "=r"(p[28]), "=r"(p[29]), "=r"(p[30]),
+          "=r"(p[31]), "=r"(p[32]), "=r"(p[33]), "=r"(p[34]), "=r"(p[35]), "=r"(p[36]),
+          "=r"(p[37]), "=r"(p[38]), "=r"(p[39]), "=r"(p[40]), "=r"(p[41]), "=r"(p[42]),
+          "=r"(p[43]), "=r"(p[44]), "=r"(p[45]), "=r"(p[46]), "=r"(p[47]), "=r"(p[48]),
+          "=r"(p[49]), "=r"(p[50]), "=r"(p[51]), "=r"(p[52]), "=r"(p[53]), "=r"(p[54]),
+          "=r"(p[55]), "=r"(p[56]), "=r"(p[57]), "=r"(p[58]), "=r"(p[59]), "=r"(p[60]),
+          "=r"(p[61]), "=r"(p[62]), "=r"(p[63]), "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]),
+          "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]), "=r"(q[10]),
+          "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15]), "=r"(q[16]),
+          "=r"(q[17]), "=r"(q[18]), "=r"(q[19]), "=r"(q[20]), "=r"(q[21]), "=r"(q[22]),
+          "=r"(q[23]), "=r"(q[24]), "=r"(q[25]), "=r"(q[26]), "=r"(q[27]), "=r"(q[28]),
+          "=r"(q[29]), "=r"(q[30]), "=r"(q[31]), "=r"(q[32]), "=r"(q[33]), "=r"(q[34]),
+          "=r"(q[35]), "=r"(q[36]), "=r"(q[37]), "=r"(q[38]), "=r"(q[39]), "=r"(q[40]),
+          "=r"(q[41]), "=r"(q[42]), "=r"(q[43]), "=r"(q[44]), "=r"(q[45]), "=r"(q[46]),
+          "=r"(q[47]), "=r"(q[48]), "=r"(q[49]), "=r"(q[50]), "=r"(q[51]), "=r"(q[52]),
+          "=r"(q[53]), "=r"(q[54]), "=r"(q[55]), "=r"(q[56]), "=r"(q[57]), "=r"(q[58]),
+          "=r"(q[59]), "=r"(q[60]), "=r"(q[61]), "=r"(q[62]), "=r"(q[63])
+        : "r"(a), "r"(a + 32), "r"(a + 64), "r"(a + 96), "r"(b), "r"(b + 32), "r"(b + 64),
+          "r"(b + 96)
+        : "memory");
+}
+
 // Register split: the launch gives 384 threads 168 registers each; the four
 // control warps keep kCtrlRegs and the eight epilogue warps take kEpiRegs,
-// which hold a warp's whole share of a tile (128 values a thread).
-constexpr int kCtrlRegs = 56, kEpiRegs = 224;
+// which hold a warp's whole share of a tile (128 values a thread) and 64 more
+// on their way from TMEM.
+constexpr int kCtrlRegs = 72, kEpiRegs = 216;
 static_assert(4 * kCtrlRegs + 8 * kEpiRegs <= 12 * 168, "register split");
 template <int R>
 __device__ __forceinline__ void reg_inc() {
@@ -241,33 +278,45 @@ __device__ __forceinline__ void reg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
 }
 
-// Adds (or stores) 16 elements of one row of TMEM into the cube: element e at
-// e0 + e * kStride of the re plane and the im plane kTile * kTile further on
-// (kStride 128: 16 columns of a tile row; 1: 16 rows of a tile column, for a
-// tile computed as its conjugate transpose).
-template <int kStride>
-__device__ __forceinline__ void store16(const Item& it, size_t e0, const int32_t (&re)[16],
-                                        const int32_t (&im)[16]) {
+// Adds into the cube.  The cube's address comes out of a table, so atomicAdd
+// would test it for shared memory at every call: 138 KB of code where these
+// make 80 KB, and an epilogue that any change to its code could slow by 2-100 %.
+// 48 small arrays in one launch 517 -> 493 us; 200 x 128, K 1024 69 -> 50 us.
+__device__ __forceinline__ void red_add(unsigned long long* p, int32_t x) {
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+                 "l"((long long)x)
+                 : "memory");
+}
+__device__ __forceinline__ void red_add(int* p, int32_t x) {
+    asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)),
+                 "r"(x)
+                 : "memory");
+}
+
+// Adds (or stores) 16 elements of one row of TMEM into the cube: columns e of
+// the re plane, kTile apart, and of the im plane kTile * kTile further on.
+__device__ __forceinline__ void store16(const Item& it, size_t e0, const uint32_t* re,
+                                        const uint32_t* im) {
     if (it.mode == MIXER_VIS_ACC_I64) {
         unsigned long long* v = reinterpret_cast<unsigned long long*>(it.vis) + e0;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            atomicAdd(v + e * kStride, (unsigned long long)(long long)re[e]);
-            atomicAdd(v + e * kStride + kTile * kTile, (unsigned long long)(long long)im[e]);
+            red_add(v + e * kTile, (int32_t)re[e]);
+            red_add(v + e * kTile + kTile * kTile, (int32_t)im[e]);
         }
     } else if (it.mode == MIXER_VIS_ACC_I32) {
         int* v = reinterpret_cast<int*>(it.vis) + e0;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            atomicAdd(v + e * kStride, re[e]);
-            atomicAdd(v + e * kStride + kTile * kTile, im[e]);
+            red_add(v + e * kTile, (int32_t)re[e]);
+            red_add(v + e * kTile + kTile * kTile, (int32_t)im[e]);
         }
     } else {
         int* v = reinterpret_cast<int*>(it.vis) + e0;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            v[e * kStride] = re[e];
-            v[e * kStride + kTile * kTile] = im[e];
+            v[e * kTile] = (int)re[e];
+            v[e * kTile + kTile * kTile] = (int)im[e];
         }
     }
 }
@@ -275,9 +324,9 @@ __device__ __forceinline__ void store16(const Item& it, size_t e0, const int32_t
 // Adds (or stores) one element of the cube, in the item's mode.
 __device__ __forceinline__ void store1(const Item& it, size_t e, int32_t x) {
     if (it.mode == MIXER_VIS_ACC_I64) {
-        atomicAdd(reinterpret_cast<unsigned long long*>(it.vis) + e, (unsigned long long)(long long)x);
+        red_add(reinterpret_cast<unsigned long long*>(it.vis) + e, x);
     } else if (it.mode == MIXER_VIS_ACC_I32) {
-        atomicAdd(reinterpret_cast<int*>(it.vis) + e, x);
+        red_add(reinterpret_cast<int*>(it.vis) + e, x);
     } else {
         reinterpret_cast<int*>(it.vis)[e] = x;
     }
@@ -299,7 +348,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int FULL = 0, EMPTY = kStages, ACCF = 2 * kStages, ACCE = 2 * kStages + 1,
-              DRAIN = 2 * kStages + 2, CLC = 2 * kStages + 3, IFULL = kItemBar0, IEMPTY = kItemBar0 + kItemSlots;
+              DRAIN = 2 * kStages + 2, CLC = 2 * kStages + 3, ACCE2 = 2 * kStages + 5,
+              IFULL = kItemBar0, IEMPTY = kItemBar0 + kItemSlots;
     auto bar = [&](int k) { return smem_u32(&bars[k]); };
 
     if (threadIdx.x == 0) {
@@ -309,6 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         mbar_init(bar(ACCF), 1);
         mbar_init(bar(ACCE), 32 * kEpiWarps);
+        mbar_init(bar(ACCE2), 32 * kEpiWarps);
         mbar_init(bar(DRAIN), 1);
         mbar_init(bar(CLC), 1);
         for (int s = 0; s < kItemSlots; ++s) {
@@ -466,12 +517,26 @@ __global__ void __launch_bounds__(kThreads, 1)
                     // 256-row B operand [Xr_j ; Xi_j]: two adjacent tiles (2 it.tail
                     // rows for a ragged block)
                     const uint64_t b = (diag && !it.tail) ? ar : sdesc(sb + 2 * kTileBytes);
+                    if (kc == 0) {
+                        // the first stage's D1 products while the epilogue reads D2
 #pragma unroll
-                    for (int kk = 0; kk < kKc / 32; ++kk) {
-                        const uint64_t o = (uint64_t)((kk * 32) >> 4);   // 32-byte K step
-                        const uint32_t acc = (kc > 0 || kk > 0) ? 1u : 0u;
-                        mma_i8(t_d1, ar + o, b + o, id1, acc);
-                        mma_i8(t_d2, ai + o, b + o, id1, acc);
+                        for (int kk = 0; kk < kKc / 32; ++kk)
+                            mma_i8(t_d1, ar + (kk * 2), b + (kk * 2), id1, kk > 0 ? 1u : 0u);
+                        if (!mbar_wait(bar(ACCE2), acc_phase ^ 1u, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+#pragma unroll
+                        for (int kk = 0; kk < kKc / 32; ++kk)
+                            mma_i8(t_d2, ai + (kk * 2), b + (kk * 2), id1, kk > 0 ? 1u : 0u);
+                    } else {
+#pragma unroll
+                        for (int kk = 0; kk < kKc / 32; ++kk) {
+                            const uint64_t o = (uint64_t)((kk * 32) >> 4);   // 32-byte K step
+                            mma_i8(t_d1, ar + o, b + o, id1, 1u);
+                            mma_i8(t_d2, ai + o, b + o, id1, 1u);
+                        }
                     }
                     tc_commit(bar(EMPTY + stage));   // stage free once these MMAs finish
                     if (++stage == kStages) {
@@ -533,32 +598,55 @@ __global__ void __launch_bounds__(kThreads, 1)
             // Im = P2 - P1.  Columns past nt are zeros (store mode writes them).
             const bool tr = it.tail && it.i != it.j;
             const int nt = it.tail ? it.tail : kTile;
-            int32_t re[kEpiChunks][16], im[kEpiChunks][16];
+            // Chunk k holds the 16 columns from 16 * (2 k + g).
+            const auto n0_of = [&](int k) { return 16 * (kEpiGroups * k + g); };
+            uint32_t re[kEpiCols], im[kEpiCols];
+            if (!it.tail) {
+                // D1 first, so that the next tile's first D1 MMAs run while D2 is read
+                const uint32_t tc = tq + 16 * g;
+                tmem_ld8_x16(tc, tc + 128, re, im);           // R1, P2
+                tc_fence_before();
+                mbar_arrive(bar(ACCE));
 #pragma unroll
-            for (int k = 0; k < kEpiChunks; ++k) {
-                const int n0 = 16 * (kEpiGroups * k + g);
-                if (n0 < nt) {
-                    uint32_t r[4][16];   // R1, P2, P1, R2
-                    tmem_ld4_x16(tq + n0, tq + nt + n0, tq + 256 + n0, tq + 256 + nt + n0, r);
+                for (int k = 0; k < kEpiChunks; k += 2) {
+                    uint32_t r[4][16];                        // P1, R2 of two chunks
+                    tmem_ld4_x16(tc + 256 + 32 * k, tc + 384 + 32 * k, tc + 288 + 32 * k,
+                                 tc + 416 + 32 * k, r);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) {
+                        re[16 * k + e] += r[2 * (e >> 4) + 1][e & 15];
+                        im[16 * k + e] = r[2 * (e >> 4)][e & 15] - im[16 * k + e];
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kEpiChunks; ++k) {
+                    const int n0 = n0_of(k);
+                    uint32_t r[4][16];                        // R1, P2, P1, R2
+                    if (n0 < nt) {
+                        tmem_ld4_x16(tq + n0, tq + nt + n0, tq + 256 + n0, tq + 256 + nt + n0, r);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) r[0][e] = r[1][e] = r[2][e] = r[3][e] = 0;
+                    }
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        re[k][e] = (int32_t)(r[0][e] + r[3][e]);
-                        im[k][e] = tr ? (int32_t)(r[1][e] - r[2][e]) : (int32_t)(r[2][e] - r[1][e]);
+                        re[16 * k + e] = r[0][e] + r[3][e];
+                        im[16 * k + e] = tr ? r[1][e] - r[2][e] : r[2][e] - r[1][e];
                     }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) re[k][e] = im[k][e] = 0;
                 }
+                tc_fence_before();
+                mbar_arrive(bar(ACCE));
             }
             tc_fence_before();
-            mbar_arrive(bar(ACCE));                  // TMEM is free for the next tile
+            mbar_arrive(bar(ACCE2));                 // TMEM is free for the next tile
             const int ncols = it.mode == MIXER_VIS_STORE_I32 ? kTile : nt;
 #pragma unroll
             for (int k = 0; k < kEpiChunks; ++k) {
-                const int n0 = 16 * (kEpiGroups * k + g);
+                const int n0 = n0_of(k);
                 if (n0 >= ncols) break;
                 if (!tr) {
-                    store16<kTile>(it, tb + (size_t)n0 * kTile + m, re[k], im[k]);
+                    store16(it, tb + (size_t)n0 * kTile + m, &re[16 * k], &im[16 * k]);
                 } else if (it.mode == MIXER_VIS_STORE_I32 &&
                            (reinterpret_cast<uintptr_t>(it.vis) & 15) == 0) {
                     // stores: a thread's 16 elements are contiguous, 4 x 16 bytes
@@ -567,8 +655,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     int4* vi = vr + kTile * kTile / 4;
 #pragma unroll
                     for (int e = 0; e < 16; e += 4) {
-                        vr[e / 4] = make_int4(re[k][e], re[k][e + 1], re[k][e + 2], re[k][e + 3]);
-                        vi[e / 4] = make_int4(im[k][e], im[k][e + 1], im[k][e + 2], im[k][e + 3]);
+                        const uint32_t *vre = &re[16 * k + e], *vim = &im[16 * k + e];
+                        vr[e / 4] = make_int4(vre[0], vre[1], vre[2], vre[3]);
+                        vi[e / 4] = make_int4(vim[0], vim[1], vim[2], vim[3]);
                     }
                 } else {
                     // row `lane` of the warp's 32 x 16 block -> pairs of rows,
@@ -579,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int pl = 0; pl < 2; ++pl) {
 #pragma unroll
                         for (int e = 0; e < 16; ++e)
-                            xs[lane * kXposeStride + e] = pl ? im[k][e] : re[k][e];
+                            xs[lane * kXposeStride + e] = pl ? im[16 * k + e] : re[16 * k + e];
                         __syncwarp();
                         const size_t pb = tb + (size_t)pl * kTile * kTile + n0 + cc;
 #pragma unroll 4
@@ -850,16 +939,15 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                     unsigned long long* v = reinterpret_cast<unsigned long long*>(args.vis) + e0;
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        atomicAdd(v + e * es, (unsigned long long)(long long)(int32_t)(r[0][e] + r[3][e]));
-                        atomicAdd(v + e * es + kTile * kTile,
-                                  (unsigned long long)(long long)(sg * (int32_t)(r[2][e] - r[1][e])));
+                        red_add(v + e * es, (int32_t)(r[0][e] + r[3][e]));
+                        red_add(v + e * es + kTile * kTile, sg * (int32_t)(r[2][e] - r[1][e]));
                     }
                 } else if (args.mode == MIXER_VIS_ACC_I32) {
                     int* v = reinterpret_cast<int*>(args.vis) + e0;
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        atomicAdd(v + e * es, (int)(r[0][e] + r[3][e]));
-                        atomicAdd(v + e * es + kTile * kTile, sg * (int)(r[2][e] - r[1][e]));
+                        red_add(v + e * es, (int32_t)(r[0][e] + r[3][e]));
+                        red_add(v + e * es + kTile * kTile, sg * (int32_t)(r[2][e] - r[1][e]));
                     }
                 } else {
                     int* v = reinterpret_cast<int*>(args.vis) + e0;
@@ -1004,7 +1092,7 @@ int xcorr_encode_maps(CUtensorMap* maps, const int8_t* planes, int32_t nant, int
 // ragged-block tiles (measured: the larger carve-out slows the int64
 // epilogue of other launches by up to 5 %).
 static int launch_smem(bool ragged) {
-    return kSmemBase + ((MIXER_XCORR_TAIL && ragged) ? kXposeBytes : 0);
+    return kSmemBase + (ragged ? kXposeBytes : 0);
 }
 
 static int set_smem_attr() {
