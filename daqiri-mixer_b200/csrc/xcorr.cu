@@ -293,16 +293,56 @@ __device__ __forceinline__ void red_add(int* p, int32_t x) {
                  : "memory");
 }
 
+// Spreads a tile's adds over the next tile's MMAs: after every kPaceCols columns
+// the warp sleeps until its share of the time has passed.  The MMAs at full
+// rate take all that one SM can read from L2 (64 bytes a clock), so operands
+// that come late are not made up for, and while the adds leave in one burst
+// the operand loads get about a third of that: 16 chunks of MMAs took 28 000
+// clocks beside the int64 adds and 19 300 beside int32 stores, against 16 400
+// alone.  One B200, without -> with: int64, 4096 x 8, K 2048 531 -> 488 us, K
+// 3072 685 -> 607, K 8192 1553 -> 1441; 1024 x 64, K 2048 298 -> 279; 640 x 48,
+// K 8192 257 -> 247; int32, 4096 x 8, K 1024 263 -> 254, K 2048 413 -> 370.
+// Shorter tiles are bound by the cube's traffic itself and are not paced.  The
+// time spread over is a tile's MMA time (1024 clocks a chunk), 1.2 times that
+// for int64 (1.0: 0-7 % slower, 0.9: 3-8 %), at most 64 x kPaceMax clocks.
+constexpr int kPaceCols = 4;
+constexpr int kPaceChunks64 = 16, kPaceChunks32 = 8;   // shortest tile paced
+constexpr int kPaceMax64 = 600, kPaceMax32 = 400;      // clocks per column
+
+struct Pace {
+    uint32_t t0, dt, due;   // start, clocks per step, clocks after t0 at which the next is due
+    __device__ __forceinline__ void begin(const Item& it) {
+        const int col = it.mode == MIXER_VIS_ACC_I64 ? min(it.nkc * 19, kPaceMax64)
+                                                     : min(it.nkc * 16, kPaceMax32);
+        dt = (uint32_t)(col * kPaceCols);
+        due = 0;
+        t0 = now();
+    }
+    __device__ __forceinline__ void step() {
+        due += dt;
+        const int32_t ahead = (int32_t)(due - (now() - t0));
+        // a quarter of the clocks left in ns: shorter than they are at any clock rate
+        if (ahead > 48) asm volatile("nanosleep.u32 %0;" ::"r"(ahead / 4) : "memory");
+    }
+    static __device__ __forceinline__ uint32_t now() {
+        uint32_t c;
+        asm volatile("mov.u32 %0, %%clock;" : "=r"(c)::"memory");
+        return c;
+    }
+};
+
 // Adds (or stores) 16 elements of one row of TMEM into the cube: columns e of
 // the re plane, kTile apart, and of the im plane kTile * kTile further on.
+template <bool kPaced>
 __device__ __forceinline__ void store16(const Item& it, size_t e0, const uint32_t* re,
-                                        const uint32_t* im) {
+                                        const uint32_t* im, Pace& pace) {
     if (it.mode == MIXER_VIS_ACC_I64) {
         unsigned long long* v = reinterpret_cast<unsigned long long*>(it.vis) + e0;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
             red_add(v + e * kTile, (int32_t)re[e]);
             red_add(v + e * kTile + kTile * kTile, (int32_t)im[e]);
+            if (kPaced && e % kPaceCols == kPaceCols - 1) pace.step();
         }
     } else if (it.mode == MIXER_VIS_ACC_I32) {
         int* v = reinterpret_cast<int*>(it.vis) + e0;
@@ -310,6 +350,7 @@ __device__ __forceinline__ void store16(const Item& it, size_t e0, const uint32_
         for (int e = 0; e < 16; ++e) {
             red_add(v + e * kTile, (int32_t)re[e]);
             red_add(v + e * kTile + kTile * kTile, (int32_t)im[e]);
+            if (kPaced && e % kPaceCols == kPaceCols - 1) pace.step();
         }
     } else {
         int* v = reinterpret_cast<int*>(it.vis) + e0;
@@ -317,6 +358,7 @@ __device__ __forceinline__ void store16(const Item& it, size_t e0, const uint32_
         for (int e = 0; e < 16; ++e) {
             v[e * kTile] = (int)re[e];
             v[e * kTile + kTile * kTile] = (int)im[e];
+            if (kPaced && e % kPaceCols == kPaceCols - 1) pace.step();
         }
     }
 }
@@ -641,12 +683,26 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_fence_before();
             mbar_arrive(bar(ACCE2));                 // TMEM is free for the next tile
             const int ncols = it.mode == MIXER_VIS_STORE_I32 ? kTile : nt;
+            const int pace_min = it.mode == MIXER_VIS_ACC_I64 ? kPaceChunks64 : kPaceChunks32;
+            Pace pace;
+            // Not in short launches, nor for the CTA's last tile, which no MMAs follow.
+            if (args.dynamic && it.nkc >= pace_min && !it.tail &&
+                __all_sync(0xffffffffu, mbar_test(bar(IFULL + islot), iphase)) &&
+                witems[islot] >= 0) {
+                pace.begin(it);
+#pragma unroll
+                for (int k = 0; k < kEpiChunks; ++k)
+                    store16<true>(it, tb + (size_t)n0_of(k) * kTile + m, &re[16 * k], &im[16 * k],
+                                  pace);
+                acc_phase ^= 1u;
+                continue;
+            }
 #pragma unroll
             for (int k = 0; k < kEpiChunks; ++k) {
                 const int n0 = n0_of(k);
                 if (n0 >= ncols) break;
                 if (!tr) {
-                    store16(it, tb + (size_t)n0 * kTile + m, &re[16 * k], &im[16 * k]);
+                    store16<false>(it, tb + (size_t)n0 * kTile + m, &re[16 * k], &im[16 * k], pace);
                 } else if (it.mode == MIXER_VIS_STORE_I32 &&
                            (reinterpret_cast<uintptr_t>(it.vis) & 15) == 0) {
                     // stores: a thread's 16 elements are contiguous, 4 x 16 bytes
