@@ -110,7 +110,9 @@ struct XcorrArgs {
     int32_t mode;
     int32_t dynamic;     // 1: one CTA per item, taken over by the running ones; 0: CTA b
                          // takes items b, b + grid, ...
-    int64_t nwork;       // nch * ntiles, or the length of `work`
+    int32_t kparts;      // items per (channel, tile), each `kpart` chunks of the range
+    int32_t kpart;
+    int64_t nwork;       // nch * ntiles * kparts, or the length of `work`
     void* vis;
     int32_t* err;
     // Batched mode (work != nullptr): per-array tensor maps, problems, work list.
@@ -139,6 +141,7 @@ struct Item {
     void* vis;
     int c, t, i, j, kbeg, kc0, nkc, mode, ntiles;
     int tail;   // rows per plane of the ragged last block on the N side (0: full tile)
+    int rows;   // rows of the MMA's M side that hold antennas
 };
 
 // Rows per plane of the last 128-row block rounded up to 16 (128 when full).
@@ -152,6 +155,15 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
     Item it;
     int nant;
     if (a.work == nullptr) {
+        it.kc0 = 0;
+        it.nkc = a.nkc;
+        if (a.kparts > 1) {           // K ranges of all tiles, one range after the other
+            const int tiles = a.nch * a.ntiles;
+            const int part = (int)w / tiles;
+            w -= part * tiles;
+            it.kc0 = part * a.kpart;
+            it.nkc = min(a.kpart, a.nkc - it.kc0);
+        }
         it.c = (int)(w / a.ntiles);
         it.t = (int)(w - (int64_t)it.c * a.ntiles);
         it.map = pmap;
@@ -159,8 +171,6 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
         nant = a.nant;
         it.vis = a.vis;
         it.kbeg = a.kbeg;
-        it.kc0 = 0;
-        it.nkc = a.nkc;
         it.mode = a.mode;
         it.ntiles = a.ntiles;
     } else {
@@ -181,6 +191,7 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
     decode_tile(it.t, it.i, it.j);
     const int r16 = tail_rows(nant);
     it.tail = (r16 < kTile && it.i == (nant - 1) / kTile) ? r16 : 0;
+    it.rows = it.i == it.j ? min(nant - it.i * kTile, kTile) : kTile;
     return it;
 }
 
@@ -702,7 +713,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int n0 = n0_of(k);
                 if (n0 >= ncols) break;
                 if (!tr) {
-                    store16<false>(it, tb + (size_t)n0 * kTile + m, &re[16 * k], &im[16 * k], pace);
+                    // rows past the last antenna would add zeros (half of a 64-element
+                    // array's adds: 64 x 64, K 256 8.6 -> 7.3 us); stores write them
+                    if (m < it.rows || it.mode == MIXER_VIS_STORE_I32)
+                        store16<false>(it, tb + (size_t)n0 * kTile + m, &re[16 * k], &im[16 * k],
+                                       pace);
                 } else if (it.mode == MIXER_VIS_STORE_I32 &&
                            (reinterpret_cast<uintptr_t>(it.vis) & 15) == 0) {
                     // stores: a thread's 16 elements are contiguous, 4 x 16 bytes
@@ -1243,6 +1258,29 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
     return MIXER_OK;
 }
 
+// K ranges per tile.  A launch with at most half as many tiles as CTAs splits
+// their K range over the idle ones, at least two chunks each: the additional
+// adds (a tile's 256 KB an item) are sent from other SMs, side by side.  Stored
+// tiles cannot be split.  One B200, whole -> split, int64: 64 x 16, K 1024 10.6
+// -> 6.6 us, K 4096 22.3 -> 8.7 us; 64 x 64, K 4096 23.4 -> 15.2 us; 200 x 16, K
+// 4096 27.9 -> 17.8 us; 256 x 20, K 8192 48.3 -> 32.7 us.  At least four or
+// eight chunks: 64 x 16, K 1024 7.4 and 9.0 us.
+constexpr int kPartChunks = 2;
+
+static void split_k(XcorrArgs& a, int32_t max_ctas) {
+    a.kparts = 1;
+    a.kpart = a.nkc;
+    int64_t ctas = sm_count();
+    if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
+    if (a.mode == MIXER_VIS_STORE_I32 || 2 * a.nwork > ctas) return;
+    int64_t parts = ctas / a.nwork;
+    if (parts > a.nkc / kPartChunks) parts = a.nkc / kPartChunks;
+    if (parts < 2) return;
+    a.kpart = (int32_t)((a.nkc + parts - 1) / parts);
+    a.kparts = (a.nkc + a.kpart - 1) / a.kpart;
+    a.nwork *= a.kparts;
+}
+
 // Grid of a launch, and how its CTAs find their items.  Round robin leaves the
 // SMs that reach their memory more slowly behind: at 1024 elements, K 1024,
 // where the cube's read-modify-write is the bound, the SMs were busy for 82 %
@@ -1285,6 +1323,7 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
     a.nkc = (int32_t)((klen + kWorkChunk - 1) / kWorkChunk);
     a.mode = mode;
     a.nwork = (int64_t)nch * a.ntiles;
+    split_k(a, max_ctas);
     a.vis = vis;
     a.err = err;
     a.tmaps = nullptr;

@@ -630,3 +630,32 @@ def test_context_long_calls(cuda, nheaps, on_device, i32):
         assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
         st = ctx.stats()
         assert st["samples"] == nheaps * tpkt and st["seq_errors"] == 0 and st["kernel_err"] == 0
+
+
+# ------------------------------------------------ K ranges split over idle SMs
+
+@pytest.mark.parametrize("nant,nch,klen,max_ctas", [
+    (40, 1, 384, 0),       # one part of two chunks at most: not split
+    (40, 1, 400, 0),       # four chunks, the last one short: two parts
+    (60, 7, 1296, 0),      # parts of unequal length
+    (70, 74, 512, 0),      # 148 items: two parts a tile
+    (70, 75, 512, 0),      # more than half the SMs: not split
+    (200, 3, 1280, 0),     # ragged tiles, plain and transposed
+    (40, 2, 2048, 7),      # parts bounded by the CTA limit
+    (40, 8, 1024, 7),      # more tiles than CTAs
+])
+def test_xcorr_k_parts(cuda, nant, nch, klen, max_ctas):
+    import torch
+    rng = np.random.default_rng(klen + nch)
+    planes = _rand_planes(rng, nch, nant, klen)
+    ref = oracle.vis_tile_pack(oracle.correlate(planes)).reshape(-1)
+    dpl = _t(planes, cuda)
+    err = _zeros(1, torch.int32, cuda)
+    for mode, dtype in ((mixer.VIS_STORE_I32, torch.int32), (mixer.VIS_ACC_I32, torch.int32),
+                        (mixer.VIS_ACC_I64, torch.int64)):
+        vis = torch.full((ref.size,), 5, dtype=dtype, device=cuda)
+        mixer.xcorr_tri(dpl, nant, nch, klen, 0, klen, mode, vis, err, max_ctas=max_ctas)
+        _sync()
+        start = 0 if mode == mixer.VIS_STORE_I32 else 5
+        assert np.array_equal(vis.cpu().numpy().astype(np.int64), ref + start), mode
+    assert int(err.item()) == 0
