@@ -194,12 +194,32 @@ def _ptr(x) -> int | None:
     raise TypeError(f"cannot take the address of {type(x)}")
 
 
+_current_raw = None   # () -> handle of torch's current stream, once torch has CUDA up
+
+
+def _bind_current_raw(torch):
+    """torch.cuda.current_stream() builds a Stream object, which took 3.2 of a
+    call's 10 us of host time; the raw handle of the current device's current
+    stream takes 0.2 us where this torch has it."""
+    global _current_raw
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device and raw:
+        _current_raw = lambda: raw(device())
+    else:
+        _current_raw = lambda: torch.cuda.current_stream().cuda_stream
+
+
 def _stream(s) -> int | None:
     if s is None:
+        if _current_raw is not None:
+            return _current_raw()
         try:
             import torch
             if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
+                handle = torch.cuda.current_stream().cuda_stream
+                _bind_current_raw(torch)
+                return handle
         except ImportError:
             pass
         return None

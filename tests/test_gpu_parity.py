@@ -659,3 +659,28 @@ def test_xcorr_k_parts(cuda, nant, nch, klen, max_ctas):
         start = 0 if mode == mixer.VIS_STORE_I32 else 5
         assert np.array_equal(vis.cpu().numpy().astype(np.int64), ref + start), mode
     assert int(err.item()) == 0
+
+
+# ------------------------------------------------- the stream a call without one uses
+
+def test_default_stream_is_torchs_current(cuda):
+    import threading
+    import torch
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    seen = {}
+
+    def thread():
+        seen["thread"] = mixer._stream(None)
+        with torch.cuda.stream(other):
+            seen["thread side"] = mixer._stream(None)
+
+    for _ in range(2):      # the first call binds, the second uses it
+        assert mixer._stream(None) == torch.cuda.current_stream().cuda_stream
+        with torch.cuda.stream(side):
+            assert mixer._stream(None) == side.cuda_stream
+            t = threading.Thread(target=thread)
+            t.start()
+            t.join()
+    assert seen == {"thread": torch.cuda.default_stream().cuda_stream,
+                    "thread side": other.cuda_stream}
+    assert mixer._stream(side) == side.cuda_stream and mixer._stream(7) == 7
