@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(256)
     const int hstride = 2 * part + tpkt;   // padded heap stride in shared memory
     const uint32_t bar = smem_u32(&bar_store);
 
+    pdl_wait();
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
@@ -156,9 +157,9 @@ extern "C" int mixer_corner_turn(const uint8_t* packets, int64_t pkt_stride, int
         MIXER_CK(cudaFuncSetAttribute(mixer::k_corner_turn,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)nant, (unsigned)ngroups, (unsigned)((nch + nchg - 1) / nchg));
-    mixer::k_corner_turn<<<grid, 256, smem, static_cast<cudaStream_t>(stream)>>>(
-        packets, pkt_stride, hdr_bytes, nant, nch, tpkt, nheaps, hg, nchg, seq0, planes, kt, k0,
-        seq_errors, err);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(mixer::launch_dependent(mixer::k_corner_turn, grid, dim3(256), smem,
+                                     static_cast<cudaStream_t>(stream), packets, pkt_stride,
+                                     hdr_bytes, nant, nch, tpkt, nheaps, hg, nchg, seq0, planes, kt,
+                                     k0, seq_errors, err));
     return MIXER_OK;
 }

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(256)
                  unsigned long long* __restrict__ grid) {
     extern __shared__ unsigned long long win[];
     __shared__ unsigned long long diag[2];
+    pdl_trigger();   // the FFT makes its twiddles beside the last CTAs
     const int t = blockIdx.x, c = blockIdx.y;
     int i, j;
     decode_tile_g(t, i, j);
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(512)
         sincospi(2.0 * (double)k / (double)G, &sn, &cs);
         tw[k] = make_float2((float)cs, (float)(-sn));
     }
+    pdl_wait();
     const long long* g = grid + (size_t)c * GG * 2;
     const int sh = 32 - logG;
     for (int q = threadIdx.x; q < GG; q += blockDim.x) {
@@ -276,6 +278,7 @@ __global__ void __launch_bounds__(1024)
         tw[k] = make_float2((float)cs, (float)(-sn));
     }
     __syncthreads();
+    pdl_wait();
     const long long* g = grid + (size_t)c * G * G * 2;
     for (int y = warp; y < G; y += nwarps) {           // rows
         float2 v[E];
@@ -336,9 +339,8 @@ int launch_fft_warp(const int64_t* grid, int32_t nch, float* img, float* vmax, f
     if (smem > 48 * 1024)
         MIXER_CK(cudaFuncSetAttribute(k_image_fft_warp<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-    k_image_fft_warp<G><<<(unsigned)nch, 1024, smem, st>>>(reinterpret_cast<const long long*>(grid),
-                                                           img, vmax, vmin);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(launch_dependent(k_image_fft_warp<G>, dim3((unsigned)nch), dim3(1024), smem, st,
+                              reinterpret_cast<const long long*>(grid), img, vmax, vmin));
     return MIXER_OK;
 }
 
@@ -402,9 +404,9 @@ extern "C" int mixer_image_fft(const int64_t* grid, int32_t nch, int32_t G, floa
     if (smem > 48 * 1024)
         MIXER_CK(cudaFuncSetAttribute(mixer::k_image_fft,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mixer::k_image_fft<<<(unsigned)nch, 512, smem, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const long long*>(grid), G, logG, img, vmax, vmin);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(mixer::launch_dependent(mixer::k_image_fft, dim3((unsigned)nch), dim3(512), smem, st,
+                                     reinterpret_cast<const long long*>(grid), G, logG, img, vmax,
+                                     vmin));
     return MIXER_OK;
 }
 

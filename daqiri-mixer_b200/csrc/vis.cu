@@ -16,6 +16,7 @@ namespace {
 
 __global__ void __launch_bounds__(256)
     k_vis_flush(int4* __restrict__ v32, longlong2* __restrict__ v64, int64_t n4) {
+    pdl_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int4 a = v32[i];
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(256)
     T* plane = out + ((size_t)c * 2 + p) * (size_t)nant * nant;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int a0 = 128 * i, b0 = 128 * j + 32 * ng;
+    pdl_wait();
     long long v[4][4];   // column w + 8 q, row lane + 32 r
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -108,9 +110,8 @@ int unpack(const int64_t* vis64, int32_t nant, int32_t nch, T* out, void* stream
     const int nt = mixer_vis_tiles(nant);
     if (2 * nt > 65535) return MIXER_EINVAL;
     dim3 grid(4, (unsigned)(2 * nt), (unsigned)nch);
-    k_vis_unpack<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const long long*>(vis64), nant, nt, out);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(launch_dependent(k_vis_unpack<T>, grid, dim3(256), 0, static_cast<cudaStream_t>(stream),
+                              reinterpret_cast<const long long*>(vis64), nant, nt, out));
     return MIXER_OK;
 }
 
@@ -124,9 +125,10 @@ extern "C" int mixer_vis_flush(int32_t* vis32, int64_t* vis64, int64_t n, void* 
     const int64_t n4 = n / 4;
     int64_t blocks = (n4 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    mixer::k_vis_flush<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<int4*>(vis32), reinterpret_cast<longlong2*>(vis64), n4);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(mixer::launch_dependent(mixer::k_vis_flush, dim3((unsigned)blocks), dim3(256), 0,
+                                     static_cast<cudaStream_t>(stream),
+                                     reinterpret_cast<int4*>(vis32),
+                                     reinterpret_cast<longlong2*>(vis64), n4));
     return MIXER_OK;
 }
 

@@ -434,6 +434,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();   // the planes, the cube and the work list are other kernels' until here
 
     if (warp < kEpiWarp0) reg_dec<kCtrlRegs>();
     if (warp == 0) {
@@ -1330,9 +1331,8 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
     a.probs = nullptr;
     a.work = nullptr;
     const int64_t grid = launch_grid(a, max_ctas);
-    k_xcorr_tri<<<(unsigned)grid, kThreads, launch_smem(nant % kTile != 0), st>>>(maps[0], maps[1],
-                                                                                  a);
-    MIXER_CK(cudaGetLastError());
+    MIXER_CK(launch_dependent(k_xcorr_tri, dim3((unsigned)grid), dim3(kThreads),
+                              launch_smem(nant % kTile != 0), st, maps[0], maps[1], a));
     return MIXER_OK;
 }
 
@@ -1351,9 +1351,9 @@ int xcorr_launch_table(const CUtensorMap* d_tmaps, const XcorrProblem* d_probs,
     a.work = d_work;
     CUtensorMap unused;
     memset(&unused, 0, sizeof(unused));
-    k_xcorr_tri<<<(unsigned)launch_grid(a, 0), kThreads, launch_smem(ragged), st>>>(unused, unused,
-                                                                                    a);
-    MIXER_CK(cudaGetLastError());
+    const int64_t grid = launch_grid(a, 0);
+    MIXER_CK(launch_dependent(k_xcorr_tri, dim3((unsigned)grid), dim3(kThreads),
+                              launch_smem(ragged), st, unused, unused, a));
     return MIXER_OK;
 }
 

@@ -684,3 +684,52 @@ def test_default_stream_is_torchs_current(cuda):
     assert seen == {"thread": torch.cuda.default_stream().cuda_stream,
                     "thread side": other.cuda_stream}
     assert mixer._stream(side) == side.cuda_stream and mixer._stream(7) == 7
+
+
+# ------------------------ dependent launches: captured, forked over streams, replayed
+
+def test_dependent_launches_captured(cuda):
+    import torch
+    nant, nch, tpkt, nheaps, G = 72, 6, 16, 24, 32
+    stride, k = 64 + 2 * nch * tpkt, nheaps * tpkt
+    rng = np.random.default_rng(5)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    n = mixer.vis_elems(nant, nch)
+
+    def buffers():
+        return dict(planes=torch.zeros((2, nch, nant, k), dtype=torch.int8, device=cuda),
+                    v32=torch.zeros(n, dtype=torch.int32, device=cuda),
+                    v64=torch.zeros(n, dtype=torch.int64, device=cuda),
+                    dump=torch.zeros((nch, 2, nant, nant), device=cuda),
+                    grid=torch.zeros((nch, G, G, 2), dtype=torch.int64, device=cuda),
+                    img=torch.zeros((nch, G, G), device=cuda))
+
+    def chain(b, st, side):
+        with torch.cuda.stream(st):
+            b["v64"].zero_()
+            mixer.corner_turn(pk, stride, 64, nant, nch, tpkt, nheaps, 0, b["planes"], k)
+            mixer.xcorr_tri(b["planes"], nant, nch, k, 0, k, mixer.VIS_ACC_I32, b["v32"])
+            mixer.vis_flush(b["v32"], b["v64"], n)
+            mixer.xcorr_tri(b["planes"], nant, nch, k, 0, k, mixer.VIS_ACC_I64, b["v64"])
+            side.wait_stream(st)
+            mixer.grid(b["v64"], nant, nch, 9, G, b["grid"])
+            mixer.image_fft(b["grid"], nch, G, b["img"])
+        with torch.cuda.stream(side):
+            mixer.vis_dump_f32(b["v64"], nant, nch, b["dump"])
+        st.wait_stream(side)
+
+    st, side = torch.cuda.Stream(), torch.cuda.Stream()
+    eager, graphed = buffers(), buffers()
+    torch.cuda.synchronize()
+    chain(eager, st, side)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        chain(graphed, st, side)
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    ref = 2 * oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    assert np.array_equal(eager["dump"].cpu().numpy(), ref.astype(np.float32))
+    for name in eager:
+        assert torch.equal(eager[name], graphed[name]), name
