@@ -110,9 +110,11 @@ struct XcorrArgs {
     int32_t mode;
     int32_t dynamic;     // 1: one CTA per item, taken over by the running ones; 0: CTA b
                          // takes items b, b + grid, ...
-    int32_t kparts;      // items per (channel, tile), each `kpart` chunks of the range
-    int32_t kpart;
-    int64_t nwork;       // nch * ntiles * kparts, or the length of `work`
+    // Single array: the first nwhole tiles are one item each, the last nsplit
+    // several, `kpart` chunks of the range each.
+    int32_t nsplit, kpart;
+    int64_t nwhole;
+    int64_t nwork;       // items
     void* vis;
     int32_t* err;
     // Batched mode (work != nullptr): per-array tensor maps, problems, work list.
@@ -157,10 +159,9 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
     if (a.work == nullptr) {
         it.kc0 = 0;
         it.nkc = a.nkc;
-        if (a.kparts > 1) {           // K ranges of all tiles, one range after the other
-            const int tiles = a.nch * a.ntiles;
-            const int part = (int)w / tiles;
-            w -= part * tiles;
+        if (w >= a.nwhole) {          // K ranges of the last tiles, one range after the other
+            const int part = (int)(w - a.nwhole) / a.nsplit;
+            w -= (int64_t)part * a.nsplit;
             it.kc0 = part * a.kpart;
             it.nkc = min(a.kpart, a.nkc - it.kc0);
         }
@@ -1259,27 +1260,37 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
     return MIXER_OK;
 }
 
-// K ranges per tile.  A launch with at most half as many tiles as CTAs splits
-// their K range over the idle ones, at least two chunks each: the additional
-// adds (a tile's 256 KB an item) are sent from other SMs, side by side.  Stored
-// tiles cannot be split.  One B200, whole -> split, int64: 64 x 16, K 1024 10.6
-// -> 6.6 us, K 4096 22.3 -> 8.7 us; 64 x 64, K 4096 23.4 -> 15.2 us; 200 x 16, K
-// 4096 27.9 -> 17.8 us; 256 x 20, K 8192 48.3 -> 32.7 us.  At least four or
-// eight chunks: 64 x 16, K 1024 7.4 and 9.0 us.
-constexpr int kPartChunks = 2;
+// K ranges of the last round's tiles.  The tiles left over after whole rounds of
+// the CTAs, when they are at most half a round, are split over all of them: the
+// MMAs get shorter by the parts, for as many more adds (a tile's 256 KB an
+// item), which other SMs send side by side.  Stored tiles cannot be split.  One
+// B200, whole -> split, int64, 128 elements: 16 channels, K 1024 13.1 -> 10.3
+// us, K 8192 45.5 -> 16.0; 164, K 4096 62.1 -> 49.8, K 16384 204 -> 132; 312, K
+// 16384 367 -> 247; 64 elements x 16, K 4096 22.3 -> 8.7.  A launch that is all
+// last round gains down to two chunks a part (64 x 16, K 1024: 6.6 us, 7.4 with
+// four, 9.0 with eight); behind whole rounds, whose adds are still under way,
+// the parts have to be longer: in two parts of four chunks 222 channels take
+// 36.1 us instead of 34.8, in two of eight 42.1 instead of 44.8.
+constexpr int kPartChunks = 2, kPartChunksBehind = 6;
 
-static void split_k(XcorrArgs& a, int32_t max_ctas) {
-    a.kparts = 1;
+static void split_last_round(XcorrArgs& a, int32_t max_ctas) {
+    const int64_t tiles = (int64_t)a.nch * a.ntiles;
+    a.nwhole = a.nwork = tiles;
+    a.nsplit = 0;
     a.kpart = a.nkc;
     int64_t ctas = sm_count();
     if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
-    if (a.mode == MIXER_VIS_STORE_I32 || 2 * a.nwork > ctas) return;
-    int64_t parts = ctas / a.nwork;
-    if (parts > a.nkc / kPartChunks) parts = a.nkc / kPartChunks;
+    const int64_t rest = tiles % ctas;
+    if (a.mode == MIXER_VIS_STORE_I32 || rest == 0) return;
+    int64_t parts = ctas / rest;
+    const int64_t most = a.nkc / (tiles == rest ? kPartChunks : kPartChunksBehind);
+    if (parts > most) parts = most;
     if (parts < 2) return;
     a.kpart = (int32_t)((a.nkc + parts - 1) / parts);
-    a.kparts = (a.nkc + a.kpart - 1) / a.kpart;
-    a.nwork *= a.kparts;
+    parts = (a.nkc + a.kpart - 1) / a.kpart;
+    a.nsplit = (int32_t)rest;
+    a.nwhole = tiles - rest;
+    a.nwork = a.nwhole + rest * parts;
 }
 
 // Grid of a launch, and how its CTAs find their items.  Round robin leaves the
@@ -1323,8 +1334,7 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
     a.kbeg = (int32_t)kbeg;
     a.nkc = (int32_t)((klen + kWorkChunk - 1) / kWorkChunk);
     a.mode = mode;
-    a.nwork = (int64_t)nch * a.ntiles;
-    split_k(a, max_ctas);
+    split_last_round(a, max_ctas);
     a.vis = vis;
     a.err = err;
     a.tmaps = nullptr;

@@ -642,7 +642,11 @@ def test_context_long_calls(cuda, nheaps, on_device, i32):
     (70, 75, 512, 0),      # more than half the SMs: not split
     (200, 3, 1280, 0),     # ragged tiles, plain and transposed
     (40, 2, 2048, 7),      # parts bounded by the CTA limit
-    (40, 8, 1024, 7),      # more tiles than CTAs
+    (40, 8, 1024, 7),      # one tile behind a whole round of the CTAs: seven in parts
+    (24, 150, 1536, 0),    # two tiles behind a whole round, in two parts of six chunks
+    (24, 150, 1408, 0),    # eleven chunks: not split
+    (24, 222, 1664, 0),    # 74 tiles behind a round, parts of seven and six chunks
+    (130, 200, 1536, 0),   # 600 items and 8 tiles in parts, taken over while they run
 ])
 def test_xcorr_k_parts(cuda, nant, nch, klen, max_ctas):
     import torch
