@@ -7,7 +7,7 @@
 // owns one (channel, lower-triangle tile), accumulates int64 sums in a small
 // shared-memory window of the baseline offsets that tile can reach, and adds
 // window cell S(d) to grid cell d and conj(S(d)) to cell -d with int64
-// atomics: the pair (b, a) carries conj(V[a][b]), so this equals the
+// atomics (stores them where the tile is the whole channel): the pair (b, a) carries conj(V[a][b]), so this equals the
 // full-square sum exactly, in any order.
 //
 // mixer_image_fft replaces cufftPlanMany/cufftExecC2C (src/rx_host_corr.cu:
@@ -50,15 +50,28 @@ __device__ __forceinline__ int pmod(int v, int g) {
 }
 
 // grid: x = tile, y = channel.  smem: windows re [ny][2 sx - 1] then im, int64.
-// Launched with 256 threads: a thread keeps one tile row m (one element a) and
-// walks every other column, four loads of each plane in flight before their
-// adds, with the column element's array position advanced instead of divided.
-__global__ void __launch_bounds__(256)
+// A thread keeps one tile row m (one element a) and walks every kGroups-th
+// column, kUnroll loads of each plane in flight before their adds, with the
+// column element's array position advanced instead of divided.
+// kWhole: the tile is the whole channel and G holds its baselines without
+// wrapping, so every grid cell is written once: no cleared grid, no global
+// atomics, no delta pass.
+// HBM-bound where the CTAs fill the SMs several times over; else a tile's chain
+// of load round trips is the bound (16 of them with 256 threads and 4 loads).
+// One B200, gridding and FFT, 256 threads and 4 loads for all -> these forms:
+// one tile a channel (kWhole, 512 threads), 32 x 85 15.4 -> 9.8 us, 128 x 128
+// 35.8 -> 20.6, 106 x 256 34.7 -> 22.3, 128 x 512 49.3 -> 49.5; few tiles (8
+// loads), 256 x 128 38.5 -> 32.9, 321 x 64 41.0 -> 34.8, 512 x 21 40.6 -> 33.3;
+// many, 8 loads would take 1024 x 256 from 397 to 409 us and 512 threads to 452.
+// A window for each warp with plain adds in place of the shared-memory atomics
+// measured 473 us there.
+template <int kThreads, int kUnroll, bool kWhole>
+__global__ void __launch_bounds__(kThreads)
     k_grid_tiles(const long long* __restrict__ vis, int nant, int ntiles, int sx, int G,
-                 unsigned long long* __restrict__ grid) {
+                 unsigned long long* __restrict__ grid, longlong2* __restrict__ prev) {
     extern __shared__ unsigned long long win[];
     __shared__ unsigned long long diag[2];
-    pdl_trigger();   // the FFT makes its twiddles beside the last CTAs
+    constexpr int kGroups = kThreads / 128;
     const int t = blockIdx.x, c = blockIdx.y;
     int i, j;
     decode_tile_g(t, i, j);
@@ -70,14 +83,15 @@ __global__ void __launch_bounds__(256)
     unsigned long long* win_im = win + ncell;
     for (int q = threadIdx.x; q < 2 * ncell; q += blockDim.x) win[q] = 0ull;
     if (threadIdx.x < 2) diag[threadIdx.x] = 0ull;
+    pdl_wait();
+    pdl_trigger();   // the FFT makes its twiddles beside the last CTAs
     __syncthreads();
-
     const long long* re = vis + (((size_t)c * ntiles + t) * 2) * 16384;
     const long long* im = re + 16384;
     const int m = threadIdx.x & 127;             // this thread's tile row
     const int a = 128 * i + m;
     const int ya = a / sx, xa = a - ya * sx;
-    // Columns n = n0, n0 + 2, ... below nlim: the array's last element and, on a
+    // Columns n = n0, n0 + kGroups, ... below nlim: the array's last element and, on a
     // diagonal tile, the row itself (the upper half is the mirror image).
     int nlim = nant - 128 * j;
     if (nlim > 128) nlim = 128;
@@ -85,15 +99,15 @@ __global__ void __launch_bounds__(256)
     if (a >= nant) nlim = 0;
     int n = threadIdx.x >> 7;
     int yb = (128 * j + n) / sx;                 // the column element's array position,
-    int xb = 128 * j + n - yb * sx;              // advanced by two columns a step
+    int xb = 128 * j + n - yb * sx;              // advanced by kGroups a step
     const int cbase = (ya - dylo) * nx + xa + sx - 1;   // cell = cbase - yb * nx - xb
 #pragma unroll 1
-    for (; n < nlim; n += 8) {
-        long long vr[4], vi[4];
-        int cell[4];
+    for (; n < nlim; n += kUnroll * kGroups) {
+        long long vr[kUnroll], vi[kUnroll];
+        int cell[kUnroll];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int nn = n + 2 * u;
+        for (int u = 0; u < kUnroll; ++u) {
+            const int nn = n + kGroups * u;
             cell[u] = -2;
             vr[u] = 0;
             vi[u] = 0;
@@ -102,14 +116,14 @@ __global__ void __launch_bounds__(256)
                 vi[u] = im[nn * 128 + m];
                 cell[u] = (a == 128 * j + nn) ? -1 : cbase - yb * nx - xb;
             }
-            xb += 2;
+            xb += kGroups;
             while (xb >= sx) {
                 xb -= sx;
                 ++yb;
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < kUnroll; ++u) {
             if (cell[u] >= 0) {
                 atomicAdd(&win_re[cell[u]], (unsigned long long)vr[u]);
                 atomicAdd(&win_im[cell[u]], (unsigned long long)vi[u]);
@@ -120,6 +134,37 @@ __global__ void __launch_bounds__(256)
         }
     }
     __syncthreads();
+    if (kWhole) {
+        // Cell d holds S(d) + conj(S(-d)), of which the window has only the one
+        // with a >= b, that is dy > 0 or dy = 0 and dx >= 0.
+        for (int q = threadIdx.x; q < G * G; q += blockDim.x) {
+            const int gy = q / G, gx = q - gy * G;
+            int dy = gy < ny + dylo ? gy : gy - G, dx = gx < sx ? gx : gx - G;
+            const bool mirror = dy < 0 || (dy == 0 && dx < 0);
+            if (mirror) {
+                dy = -dy;
+                dx = -dx;
+            }
+            longlong2 v = make_longlong2(0, 0);
+            if (dy == 0 && dx == 0) {
+                v = make_longlong2((long long)diag[0], (long long)diag[1]);
+            } else if (dy < ny + dylo && dx < sx && dx > -sx) {
+                const int cell = (dy - dylo) * nx + dx + sx - 1;
+                v.x = (long long)win_re[cell];
+                v.y = (long long)win_im[cell];
+                if (mirror) v.y = -v.y;
+            }
+            const size_t o = (size_t)c * G * G + q;
+            if (prev) {
+                const longlong2 p = prev[o];
+                prev[o] = v;
+                v.x -= p.x;
+                v.y -= p.y;
+            }
+            reinterpret_cast<longlong2*>(grid)[o] = v;
+        }
+        return;
+    }
     unsigned long long* gc = grid + (size_t)c * G * G * 2;
     for (int q = threadIdx.x; q < ncell; q += blockDim.x) {
         const unsigned long long sr = win_re[q], si = win_im[q];
@@ -137,6 +182,23 @@ __global__ void __launch_bounds__(256)
         atomicAdd(&gc[1], diag[1]);
     }
 }
+
+template <int kThreads, int kUnroll, bool kWhole>
+int launch_grid_tiles(dim3 g, size_t smem, cudaStream_t st, const int64_t* vis64, int32_t nant, int nt,
+                      int32_t side_x, int32_t G, int64_t* grid, int64_t* prev) {
+    const auto kernel = k_grid_tiles<kThreads, kUnroll, kWhole>;
+    if (smem > 48 * 1024)
+        MIXER_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MIXER_CK(launch_dependent(kernel, g, dim3(kThreads), smem, st,
+                              reinterpret_cast<const long long*>(vis64), nant, nt, side_x, G,
+                              reinterpret_cast<unsigned long long*>(grid),
+                              reinterpret_cast<longlong2*>(prev)));
+    return MIXER_OK;
+}
+
+// Up to this many tiles in a launch (seven an SM) eight loads a thread pay:
+// 480 tiles 45.1 -> 41.0 us, 1920 the same.
+constexpr int64_t kGridFewTiles = 7 * 148;
 
 // grid = grid - prev, prev = old grid (delta imaging), n int64 values.
 __global__ void k_grid_delta(long long* __restrict__ grid, long long* __restrict__ prev, int64_t n) {
@@ -369,16 +431,19 @@ extern "C" int mixer_grid(const int64_t* vis64, int32_t nant, int32_t nch, int32
     const int nt = mixer_vis_tiles(nant);
     const size_t smem = mixer::grid_smem_bytes(nant, side_x);
     if (smem > mixer::kGridSmemMax) return MIXER_EINVAL;
-    if (smem > 48 * 1024)
-        MIXER_CK(cudaFuncSetAttribute(mixer::k_grid_tiles,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    dim3 g((unsigned)nt, (unsigned)nch);
+    const int rows = (nant + side_x - 1) / side_x;
+    const uintptr_t both = reinterpret_cast<uintptr_t>(grid) | reinterpret_cast<uintptr_t>(prev);
+    if (nt == 1 && G >= 2 * side_x - 1 && G >= 2 * rows - 1 && both % 16 == 0)
+        return mixer::launch_grid_tiles<512, 4, true>(g, smem, st, vis64, nant, nt, side_x, G, grid,
+                                                      prev);
     const size_t gbytes = (size_t)nch * G * G * 2 * sizeof(int64_t);
     MIXER_CK(cudaMemsetAsync(grid, 0, gbytes, st));
-    dim3 g((unsigned)nt, (unsigned)nch);
-    mixer::k_grid_tiles<<<g, 256, smem, st>>>(reinterpret_cast<const long long*>(vis64), nant, nt,
-                                              side_x, G,
-                                              reinterpret_cast<unsigned long long*>(grid));
-    MIXER_CK(cudaGetLastError());
+    const auto launch = (int64_t)nt * nch <= mixer::kGridFewTiles
+                            ? mixer::launch_grid_tiles<256, 8, false>
+                            : mixer::launch_grid_tiles<256, 4, false>;
+    const int rc = launch(g, smem, st, vis64, nant, nt, side_x, G, grid, nullptr);
+    if (rc != MIXER_OK) return rc;
     if (prev) {
         const int64_t n = (int64_t)nch * G * G * 2;
         int64_t blocks = (n + 255) / 256;
@@ -448,7 +513,7 @@ extern "C" int mixer_image_noalloc(const int64_t* vis64, int32_t nant, int32_t n
     int64_t* grid = nullptr;
     int rc = mixer::noalloc_grid_address(&grid);
     if (rc != MIXER_OK) return rc;
-    // mixer_grid clears the cells it uses on `stream` before adding into them.
+    // mixer_grid clears or overwrites the cells it uses on `stream`.
     rc = mixer_grid(vis64, nant, nch, side_x, G, grid, nullptr, stream);
     if (rc != MIXER_OK) return rc;
     return mixer_image_fft(grid, nch, G, img, vmax, vmin, stream);

@@ -182,7 +182,7 @@ int mixer_image_fft(const int64_t* grid, int32_t nch, int32_t G, float* img,
  *     another driver-API context, or calling again after cudaDeviceReset, is
  *     not supported: the kept address belongs to the first primary context.
  *   - All calls share the one array and it keeps the previous call's
- *     contents; each call clears it on `stream` before gridding.  Calls whose
+ *     contents; each call clears or overwrites what it uses on `stream`.  Calls whose
  *     work overlaps on the GPU (different streams, or several host threads)
  *     race on the array and must be serialised by the caller.
  * vis64 / img / vmax / vmin as for mixer_grid and mixer_image_fft. */

@@ -642,7 +642,7 @@ def test_context_long_calls(cuda, nheaps, on_device, i32):
     (70, 75, 512, 0),      # more than half the SMs: not split
     (200, 3, 1280, 0),     # ragged tiles, plain and transposed
     (40, 2, 2048, 7),      # parts bounded by the CTA limit
-    (40, 8, 1024, 7),      # one tile behind a whole round of the CTAs: seven in parts
+    (40, 8, 1024, 7),      # one tile behind a round of seven CTAs, too short to split
     (24, 150, 1536, 0),    # two tiles behind a whole round, in two parts of six chunks
     (24, 150, 1408, 0),    # eleven chunks: not split
     (24, 222, 1664, 0),    # 74 tiles behind a round, parts of seven and six chunks
@@ -737,3 +737,36 @@ def test_dependent_launches_captured(cuda):
     assert np.array_equal(eager["dump"].cpu().numpy(), ref.astype(np.float32))
     for name in eager:
         assert torch.equal(eager[name], graphed[name]), name
+
+
+# -------------------------------------------- the forms of the gridding kernel
+
+@pytest.mark.parametrize("nant,side,G,nch,shift", [
+    (128, 16, 31, 3, 0),     # one tile, the grid just holds its baselines: written whole
+    (128, 16, 30, 3, 0),     # one less: baselines wrap
+    (128, 16, 32, 3, 8),     # grids on an 8-byte boundary
+    (7, 9, 18, 2, 0),        # array wider than its elements
+    (90, 1, 179, 2, 0),      # one column
+    (129, 16, 32, 2, 0),     # three tiles
+    (130, 12, 32, 345, 0),   # 1035 tiles, the last launch with eight loads a thread
+    (130, 12, 32, 346, 0),   # 1038 tiles
+])
+def test_grid_forms(cuda, nant, side, G, nch, shift):
+    import torch
+    rng = np.random.default_rng(nant)
+    planes = rng.integers(-128, 128, size=(2, nch, nant, 16), dtype=np.int8)
+    full = oracle.correlate(planes)
+    vis = _t(oracle.vis_tile_pack(full).reshape(-1), cuda)
+    ref = oracle.grid(full, side, G)
+    n, off = nch * G * G * 2, shift // 8
+    grid = torch.full((n + 2,), 7, dtype=torch.int64, device=cuda)[off:off + n]
+    mixer.grid(vis, nant, nch, side, G, grid)
+    _sync()
+    assert np.array_equal(grid.cpu().numpy().reshape(ref.shape), ref)
+    old = rng.integers(-1000, 1000, size=n)
+    prev = torch.full((n + 2,), 0, dtype=torch.int64, device=cuda)[off:off + n]
+    prev.copy_(_t(old, cuda))
+    mixer.grid(vis, nant, nch, side, G, grid, prev)
+    _sync()
+    assert np.array_equal(grid.cpu().numpy(), ref.reshape(-1) - old)
+    assert np.array_equal(prev.cpu().numpy(), ref.reshape(-1))
