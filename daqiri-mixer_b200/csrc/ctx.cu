@@ -212,15 +212,57 @@ extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     return MIXER_OK;
 }
 
+// Zeroes a context's state in one launch; four memsets took as long as anything
+// else in a small array's dump.  One B200, reset to image: 30 elements x 64
+// channels 34.4 -> 26.3 us, 79 x 85 63.0 -> 56.8, 256 x 128 757 -> 753.  A cube
+// of 500 MB is left to the memset (498 us, 508 with this kernel).  Regions are
+// multiples of 16 bytes; end[k] is their running total in 16-byte vectors.
+constexpr int64_t kZeroMax = 128 << 20;
+struct ZeroRegions {
+    uint4* p[3];
+    int64_t end[3];
+    int n;
+    uint32_t* word[2];
+    void add(void* q, int64_t bytes) {
+        const int64_t before = n ? end[n - 1] : 0;
+        p[n] = static_cast<uint4*>(q);
+        for (int k = n++; k < 3; ++k) end[k] = before + bytes / 16;
+    }
+};
+static __global__ void __launch_bounds__(512) k_zero(const ZeroRegions z) {
+    mixer::pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x < 2) *z.word[threadIdx.x] = 0u;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < z.end[2]; q += step) {
+        const int k = q < z.end[0] ? 0 : (q < z.end[1] ? 1 : 2);
+        z.p[k][q - (k ? z.end[k - 1] : 0)] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
 extern "C" int mixer_reset(mixer_ctx* c, void* stream) {
     if (!c) return MIXER_EINVAL;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    MIXER_CK(cudaMemsetAsync(c->vis64, 0, (size_t)c->vis_elems * sizeof(int64_t), st));
-    if (c->vis32) MIXER_CK(cudaMemsetAsync(c->vis32, 0, (size_t)c->vis_elems * sizeof(int32_t), st));
-    MIXER_CK(cudaMemsetAsync(c->grid_prev, 0,
-                             (size_t)c->d.nch * c->d.grid * c->d.grid * 2 * sizeof(int64_t), st));
-    MIXER_CK(cudaMemsetAsync(c->d_seq_err, 0, sizeof(uint32_t), st));
-    MIXER_CK(cudaMemsetAsync(c->d_err, 0, sizeof(int32_t), st));
+    ZeroRegions z = {};
+    const struct {
+        void* p;
+        int64_t bytes;
+    } state[3] = {
+        {c->vis64, c->vis_elems * (int64_t)sizeof(int64_t)},
+        {c->vis32, c->vis_elems * (int64_t)sizeof(int32_t)},
+        {c->grid_prev, (int64_t)c->d.nch * c->d.grid * c->d.grid * 2 * (int64_t)sizeof(int64_t)}};
+    for (const auto& r : state) {
+        if (!r.p) continue;
+        if (r.bytes > kZeroMax)
+            MIXER_CK(cudaMemsetAsync(r.p, 0, (size_t)r.bytes, st));
+        else
+            z.add(r.p, r.bytes);
+    }
+    z.word[0] = reinterpret_cast<uint32_t*>(c->d_seq_err);
+    z.word[1] = reinterpret_cast<uint32_t*>(c->d_err);
+    int64_t blocks = (z.end[2] + 511) / 512;
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    if (blocks < 1) blocks = 1;
+    MIXER_CK(mixer::launch_dependent(k_zero, dim3((unsigned)blocks), dim3(512), 0, st, z));
     c->samples = 0;
     c->i32_samples = 0;
     return MIXER_OK;

@@ -770,3 +770,40 @@ def test_grid_forms(cuda, nant, side, G, nch, shift):
     _sync()
     assert np.array_equal(grid.cpu().numpy(), ref.reshape(-1) - old)
     assert np.array_equal(prev.cpu().numpy(), ref.reshape(-1))
+
+
+# ------------------------------------------------------ a context's state zeroed
+
+@pytest.mark.parametrize("i32", [False, True])       # with the int32 cube or without
+@pytest.mark.parametrize("nant,nch", [(3, 1), (140, 5), (1000, 20)])   # 190 MB: by memset
+def test_context_reset(cuda, nant, nch, i32):
+    import torch
+    tpkt, nheaps, G = 16, 2, 16
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(nant)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=32, grid=G,
+                            pkt_stride=stride, max_heaps=nheaps) as ctx:
+        img = torch.zeros(nch * G * G, device=cuda)
+        out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+        images = []
+        for _ in range(2):              # the second pass starts from what the first left
+            if i32:
+                ctx.correlate_i32(pk, nheaps, 5)      # left in the int32 cube
+            ctx.correlate(pk, nheaps, 5)
+            ctx.image(img, delta=True)
+            ctx.reset()
+            ctx.integrate()
+            ctx.read_vis_i64(out)
+            _sync()
+            assert int(out.abs().max()) == 0
+            assert ctx.stats() == {"samples": 0, "seq_errors": 0, "kernel_err": 0}
+            ctx.correlate(pk, nheaps, 5)
+            ctx.read_vis_i64(out)
+            ctx.image(img, delta=True)
+            _sync()
+            assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
+            images.append(img.clone())
+        # the delta image starts anew after a reset
+        assert torch.equal(images[0], images[1])
