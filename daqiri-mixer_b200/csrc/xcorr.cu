@@ -20,7 +20,7 @@
 // 16 rows per plane (N = 2 r16): tile (nb-1, j < nb-1) is computed as its
 // conjugate transpose, A = block j and B = [Xr_nb-1 ; Xi_nb-1] (r16 rows
 // each, one TMA box over both planes), and written back transposed; tile
-// (nb-1, nb-1) keeps A = its own block.  Operands come from the corner-turned
+// (nb-1, nb-1) has its own block on both sides (own_rows).  Operands come from the corner-turned
 // planes [2][C][N][kt] through 4-D TMA tensor loads (128-byte swizzle,
 // 128 x 128-byte boxes)
 // into a 3-deep shared-memory ring.  One elected thread issues all
@@ -145,6 +145,30 @@ struct Item {
     int tail;   // rows per plane of the ragged last block on the N side (0: full tile)
     int rows;   // rows of the MMA's M side that hold antennas
 };
+
+// A ragged block's diagonal tile has its block for both operands.  Where it pays
+// (own_rows) no 128-row A is loaded: the MMAs read A from B's rows, Xr from
+// the first on and Xi from row it.tail on (the M rows past it.tail are whatever
+// lies there, and not added; stores want zeros there and keep the 128-row A),
+// and a stage holds several K steps.  Arrays of one block: 32 elements x 256
+// channels, K 512 8.9 -> 8.0 us, K 4096 35.5 -> 28.1; 27 x 85, K 5952 26.2 ->
+// 20.4; 64 x 592, K 1024 31.4 -> 28.4.  Behind other blocks only long ranges
+// gain: 200 x 128, K 4096 76.0 -> 72.6, but 300 x 85, K 1024 48.7 -> 50.6.
+constexpr int kOwnChunks = 12;
+__device__ __forceinline__ bool own_rows(const Item& it) {
+    return it.tail && it.i == it.j && (it.i == 0 || it.nkc >= kOwnChunks) &&
+           it.mode != MIXER_VIS_STORE_I32;
+}
+// K steps of such a tile in a stage: all, if they fit, else what fits, at most 8
+// and a third of them (40 x 128, K 1024 with five and three 9.6 us, in twos 9.0).
+__device__ __forceinline__ int own_steps(int r16, int steps) {
+    const int fit = r16 <= 32 ? 8 : r16 <= 48 ? 5 : r16 <= 64 ? 4 : r16 <= 80 ? 3 : 2;
+    return steps <= fit ? steps : max(1, min(fit, steps / 3));
+}
+static_assert(8 * 2 * 32 * kKc <= kStageBytes && 5 * 2 * 48 * kKc <= kStageBytes &&
+                  4 * 2 * 64 * kKc <= kStageBytes && 3 * 2 * 80 * kKc <= kStageBytes &&
+                  2 * 2 * 112 * kKc <= kStageBytes,
+              "K steps of a ragged diagonal tile in a stage");
 
 // Rows per plane of the last 128-row block rounded up to 16 (128 when full).
 __host__ __device__ __forceinline__ int tail_rows(int nant) {
@@ -477,7 +501,30 @@ __global__ void __launch_bounds__(kThreads, 1)
                                                : (diag ? 2 * kTileBytes : 4 * kTileBytes);
                 // A block: block j for a transposed ragged tile, else block i
                 const int ia = (it.tail && !diag) ? it.j : it.i;
-                for (int kc = 0; kc < it.nkc * kSubPerChunk; ++kc) {
+                const bool own = own_rows(it);
+                if (own) {
+                    const int steps = it.nkc * kSubPerChunk, per = own_steps(it.tail, steps);
+                    const uint32_t each = 2 * it.tail * kKc;
+                    for (int kc = 0; kc < steps; kc += per) {
+                        if (!mbar_wait(bar(EMPTY + stage), phase ^ 1u, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
+                        const int n = min(per, steps - kc);
+                        const uint32_t fb = bar(FULL + stage);
+                        mbar_expect_tx(fb, n * each);
+                        for (int u = 0; u < n; ++u)
+                            tma_load_4d(base + stage * kStageBytes + u * each, it.map_tail, fb,
+                                        it.kbeg + it.kc0 * kWorkChunk + (kc + u) * kKc,
+                                        it.i * kTile, it.c, 0);
+                        ++issued;
+                        if (++stage == kStages) {
+                            stage = 0;
+                            phase ^= 1u;
+                        }
+                    }
+                }
+                for (int kc = 0; !own && kc < it.nkc * kSubPerChunk; ++kc) {
                     if (!mbar_wait(bar(EMPTY + stage), phase ^ 1u, abort_flag)) {
                         ok = false;
                         break;
@@ -560,7 +607,39 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 }
                 tc_fence_after();
-                for (int kc = 0; kc < it.nkc * kSubPerChunk; ++kc) {
+                const bool own = own_rows(it);
+                if (own) {
+                    const int steps = it.nkc * kSubPerChunk, per = own_steps(it.tail, steps);
+                    const uint64_t each = (uint64_t)((2 * it.tail * kKc) >> 4);
+                    if (!mbar_wait(bar(ACCE2), acc_phase ^ 1u, abort_flag)) ok = false;
+                    tc_fence_after();
+                    for (int kc = 0; ok && kc < steps; kc += per) {
+                        if (!mbar_wait(bar(FULL + stage), phase, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        uint64_t b = sdesc(base + stage * kStageBytes);
+                        const uint64_t im = (uint64_t)((it.tail * kKc) >> 4);
+                        const int n = min(per, steps - kc);
+#pragma unroll 1
+                        for (int u = 0; u < n; ++u, b += each) {
+                            const uint32_t acc = kc + u > 0 ? 1u : 0u;
+#pragma unroll
+                            for (int kk = 0; kk < kKc / 32; ++kk) {
+                                mma_i8(t_d1, b + (kk * 2), b + (kk * 2), id1, kk > 0 ? 1u : acc);
+                                mma_i8(t_d2, b + im + (kk * 2), b + (kk * 2), id1,
+                                       kk > 0 ? 1u : acc);
+                            }
+                        }
+                        tc_commit(bar(EMPTY + stage));
+                        if (++stage == kStages) {
+                            stage = 0;
+                            phase ^= 1u;
+                        }
+                    }
+                }
+                for (int kc = 0; !own && kc < it.nkc * kSubPerChunk; ++kc) {
                     if (!mbar_wait(bar(FULL + stage), phase, abort_flag)) {
                         ok = false;
                         break;

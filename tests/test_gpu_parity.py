@@ -807,3 +807,25 @@ def test_context_reset(cuda, nant, nch, i32):
             images.append(img.clone())
         # the delta image starts anew after a reset
         assert torch.equal(images[0], images[1])
+
+
+# --------------------------- a ragged diagonal tile with both operands from one box
+
+@pytest.mark.parametrize("nant", [16, 17, 33, 50, 65, 81, 97, 112, 144, 200])
+@pytest.mark.parametrize("klen", [80, 512, 1152, 1408, 1520, 2480])   # 1 to 20 chunks
+def test_xcorr_ragged_diagonal(cuda, nant, klen):
+    import torch
+    nch = 75 if nant <= 128 else 50       # one item a tile, no K ranges
+    rng = np.random.default_rng(nant)
+    planes = _rand_planes(rng, nch, nant, klen)
+    ref = oracle.vis_tile_pack(oracle.correlate(planes)).reshape(-1)
+    dpl = _t(planes, cuda)
+    err = _zeros(1, torch.int32, cuda)
+    for mode, dtype in ((mixer.VIS_STORE_I32, torch.int32), (mixer.VIS_ACC_I32, torch.int32),
+                        (mixer.VIS_ACC_I64, torch.int64)):
+        vis = torch.full((ref.size,), 3, dtype=dtype, device=cuda)
+        mixer.xcorr_tri(dpl, nant, nch, klen, 0, klen, mode, vis, err)
+        _sync()
+        start = 0 if mode == mixer.VIS_STORE_I32 else 3
+        assert np.array_equal(vis.cpu().numpy().astype(np.int64), ref + start), mode
+    assert int(err.item()) == 0
