@@ -12,13 +12,14 @@
 // items by s (better balance over the persistent grid) at the cost of s
 // int64 read-modify-write epilogues per tile; integer sums are exact in any
 // order, so every split gives bit-identical visibilities.
-// Triangle schedule: items ordered longest-first (the static round-robin over
-// CTAs then approximates longest-processing-time scheduling) or in natural
-// array / channel / tile order (L2 locality of a channel's operands).
+// Triangle schedule: items ordered longest-first (taken in list order this is
+// longest-processing-time scheduling) or in natural array / channel / tile
+// order (L2 locality of a channel's operands).
 // The autotuner times candidate plans on the caller's own buffers, each in an
 // A-B-B-A pairing with the incumbent, and keeps a change only for a clear gain;
-// the chosen launch can be captured once into a CUDA graph and replayed.  This has no counterpart in the reference, which launches one
-// fixed-shape kernel per V-update (src/rx_host_corr.cu:167).
+// the chosen launch can be captured once into a CUDA graph and replayed.  This
+// has no counterpart in the reference, which launches one fixed-shape kernel
+// per V-update (src/rx_host_corr.cu:167).
 #include <algorithm>
 #include <cstring>
 #include <vector>
