@@ -162,6 +162,25 @@ static bool alloc_long_planes(mixer_ctx* c) {
     return true;
 }
 
+// Device memory for a buffer made on first use.  When there is none left, planes
+// longer than max_heaps are given back for it.
+static int alloc_late(mixer_ctx* c, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && c->kt_planes > c->kt_max) {
+        cudaGetLastError();
+        MIXER_CK(cudaDeviceSynchronize());   // launches may still be reading them
+        cudaFree(c->planes);
+        c->planes = nullptr;
+        c->kt_planes = 0;
+        MIXER_CK(cudaMalloc(&c->planes, (size_t)2 * c->d.nch * c->d.nant * c->kt_max));
+        c->kt_planes = c->kt_max;
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    MIXER_CK(e);
+    return MIXER_OK;
+}
+
 extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     if (!out) return MIXER_EINVAL;
     *out = nullptr;
@@ -276,6 +295,7 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
     if (!c || !packets || nheaps <= 0) return MIXER_EINVAL;
     const mixer_array_desc& d = c->d;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!c->planes) return MIXER_ENOMEM;   // given back, and no room for short ones either
     const uint8_t* src = static_cast<const uint8_t*>(packets);
     const int64_t heap_bytes = (int64_t)d.nant * d.pkt_stride;
     const int64_t most =
@@ -289,7 +309,10 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
         const uint8_t* dev_chunk = chunk;
         if (!on_device) {
             const int s = c->cur;
-            if (!c->stage[s]) MIXER_CK(cudaMalloc(&c->stage[s], c->stage_bytes));
+            if (!c->stage[s]) {
+                const int rc = alloc_late(c, reinterpret_cast<void**>(&c->stage[s]), c->stage_bytes);
+                if (rc != MIXER_OK) return rc;
+            }
             if (c->stage_used[s]) MIXER_CK(cudaStreamWaitEvent(c->copy_stream, c->stage_free[s], 0));
             MIXER_CK(cudaMemcpyAsync(c->stage[s], chunk, (size_t)nh * heap_bytes,
                                      cudaMemcpyHostToDevice, c->copy_stream));
@@ -326,7 +349,9 @@ extern "C" int mixer_correlate_i32(mixer_ctx* c, const void* packets, int64_t nh
     if (!c || nheaps <= 0) return MIXER_EINVAL;
     if (c->i32_samples + nheaps * c->d.tpkt > MIXER_KMAX_I32) return MIXER_EOVERFLOW;
     if (!c->vis32) {
-        MIXER_CK(cudaMalloc(&c->vis32, (size_t)c->vis_elems * sizeof(int32_t)));
+        const int rc = alloc_late(c, reinterpret_cast<void**>(&c->vis32),
+                                  (size_t)c->vis_elems * sizeof(int32_t));
+        if (rc != MIXER_OK) return rc;
         MIXER_CK(cudaMemsetAsync(c->vis32, 0, (size_t)c->vis_elems * sizeof(int32_t),
                                  static_cast<cudaStream_t>(stream)));
     }
@@ -351,8 +376,10 @@ extern "C" int mixer_dump(mixer_ctx* c, float* out, int32_t out_on_device, void*
     if (!c || !out) return MIXER_EINVAL;
     const size_t n = (size_t)c->d.nch * 2 * c->d.nant * c->d.nant;
     if (out_on_device) return mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, out, stream);
-    if (!c->dump_dev) MIXER_CK(cudaMalloc(&c->dump_dev, n * sizeof(float)));
-    int rc = mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, c->dump_dev, stream);
+    int rc = c->dump_dev ? MIXER_OK
+                         : alloc_late(c, reinterpret_cast<void**>(&c->dump_dev), n * sizeof(float));
+    if (rc != MIXER_OK) return rc;
+    rc = mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, c->dump_dev, stream);
     if (rc != MIXER_OK) return rc;
     MIXER_CK(cudaMemcpyAsync(out, c->dump_dev, n * sizeof(float), cudaMemcpyDeviceToHost,
                              static_cast<cudaStream_t>(stream)));
@@ -393,8 +420,11 @@ extern "C" int mixer_read_vis_i64(mixer_ctx* c, int64_t* out, int32_t full_squar
     }
     const size_t n = (size_t)c->d.nch * 2 * c->d.nant * c->d.nant;
     if (out_on_device) return mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, out, stream);
-    if (!c->unpack_dev) MIXER_CK(cudaMalloc(&c->unpack_dev, n * sizeof(int64_t)));
-    int rc = mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, c->unpack_dev, stream);
+    int rc = c->unpack_dev
+                 ? MIXER_OK
+                 : alloc_late(c, reinterpret_cast<void**>(&c->unpack_dev), n * sizeof(int64_t));
+    if (rc != MIXER_OK) return rc;
+    rc = mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, c->unpack_dev, stream);
     if (rc != MIXER_OK) return rc;
     MIXER_CK(cudaMemcpyAsync(out, c->unpack_dev, n * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     return MIXER_OK;

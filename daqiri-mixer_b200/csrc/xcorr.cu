@@ -169,6 +169,11 @@ static_assert(8 * 2 * 32 * kKc <= kStageBytes && 5 * 2 * 48 * kKc <= kStageBytes
                   4 * 2 * 64 * kKc <= kStageBytes && 3 * 2 * 80 * kKc <= kStageBytes &&
                   2 * 2 * 112 * kKc <= kStageBytes,
               "K steps of a ragged diagonal tile in a stage");
+// The M rows past the block reach furthest beyond a stage with 32 rows (8 K
+// steps fill it): behind the last stage they read the barriers and the
+// transpose area, which every launch with a ragged array has.
+static_assert((7 * 2 * 32 + 32 + kTile) * kKc - kStageBytes <= kBarBytes + kXposeBytes,
+              "rows past a ragged block stay inside the launch's shared memory");
 
 // Rows per plane of the last 128-row block rounded up to 16 (128 when full).
 __host__ __device__ __forceinline__ int tail_rows(int nant) {

@@ -829,3 +829,31 @@ def test_xcorr_ragged_diagonal(cuda, nant, klen):
         start = 0 if mode == mixer.VIS_STORE_I32 else 3
         assert np.array_equal(vis.cpu().numpy().astype(np.int64), ref + start), mode
     assert int(err.item()) == 0
+
+
+def test_context_gives_long_planes_back(cuda):
+    """A buffer made on first use that no longer fits takes the long planes' place."""
+    import torch
+    nant, nch, tpkt, nheaps = 1000, 20, 16, 2
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(3)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    torch.cuda.empty_cache()
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=32, grid=64,
+                            pkt_stride=stride, max_heaps=nheaps) as ctx:
+        ctx.correlate(pk, nheaps)
+        _sync()
+        # leave 100 MB: less than the 160 MB dump, which the 655 MB planes make room for
+        fill = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (100 << 20)), dtype=torch.uint8,
+                           device=cuda)
+        dump = np.zeros(ref.shape, dtype=np.float32)
+        ctx.dump(dump, on_device=False)
+        _sync()
+        assert np.array_equal(dump, ref.astype(np.float32))
+        ctx.correlate(pk, nheaps)                      # with the short planes
+        ctx.dump(dump, on_device=False)
+        _sync()
+        assert np.array_equal(dump, (2 * ref).astype(np.float32))
+        del fill
+    torch.cuda.empty_cache()
