@@ -196,9 +196,9 @@ int launch_grid_tiles(dim3 g, size_t smem, cudaStream_t st, const int64_t* vis64
     return MIXER_OK;
 }
 
-// Up to this many tiles in a launch (seven an SM) eight loads a thread pay:
-// 480 tiles 45.1 -> 41.0 us, 1920 the same.
-constexpr int64_t kGridFewTiles = 7 * 148;
+// Up to this many tiles in a launch (four an SM) eight loads a thread pay:
+// 480 tiles 45.1 -> 41.0 us, 576 43.0 -> 37.4; 600 48.7 -> 50.3, 768 65.4 -> 71.5.
+constexpr int64_t kGridFewTiles = 4 * 148;
 
 // grid = grid - prev, prev = old grid (delta imaging), n int64 values.
 __global__ void k_grid_delta(long long* __restrict__ grid, long long* __restrict__ prev, int64_t n) {

@@ -748,8 +748,8 @@ def test_dependent_launches_captured(cuda):
     (7, 9, 18, 2, 0),        # array wider than its elements
     (90, 1, 179, 2, 0),      # one column
     (129, 16, 32, 2, 0),     # three tiles
-    (130, 12, 32, 345, 0),   # 1035 tiles, the last launch with eight loads a thread
-    (130, 12, 32, 346, 0),   # 1038 tiles
+    (130, 12, 32, 197, 0),   # 591 tiles, the last launch with eight loads a thread
+    (130, 12, 32, 198, 0),   # 594 tiles
 ])
 def test_grid_forms(cuda, nant, side, G, nch, shift):
     import torch
