@@ -783,7 +783,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int pace_min = it.mode == MIXER_VIS_ACC_I64 ? kPaceChunks64 : kPaceChunks32;
             Pace pace;
             // Not in short launches, nor for the CTA's last tile, which no MMAs follow.
-            if (args.dynamic && it.nkc >= pace_min && !it.tail &&
+            const bool many = args.dynamic || args.nwork > 4 * (int64_t)gridDim.x;
+            if (many && it.nkc >= pace_min && !it.tail &&
                 __all_sync(0xffffffffu, mbar_test(bar(IFULL + islot), iphase)) &&
                 witems[islot] >= 0) {
                 pace.begin(it);
@@ -1385,11 +1386,15 @@ static void split_last_round(XcorrArgs& a, int32_t max_ctas) {
 // K 1024 457 -> 410 us; 640 x 48 (4.9 items an SM) the same.  Below four items
 // an SM there is little to even out, and which SMs get the last round's items
 // matters more: 256 x 128 (2.6 an SM), K 1024 55 -> 57 us, so those stay round
-// robin.  Table launches hold items of different lengths and are always taken
+// robin.  So do int32 stores, which wait for no memory and gain from CTAs that
+// keep in step on a channel's row blocks: taken over -> round robin, 971 x 32, K
+// 192 50.1 -> 44.2 us, 640 x 48, K 1024 55 -> 42, 4096 x 8, K 512 142 -> 136, but
+// 1024 x 64, K 256 60.8 -> 64.8.  Table launches hold items of different lengths and are always taken
 // over; a launch with a CTA limit cannot be, since its grid would be the items.
 static int64_t launch_grid(XcorrArgs& a, int32_t max_ctas) {
     const int64_t sms = sm_count();
-    a.dynamic = max_ctas <= 0 && a.nwork <= INT32_MAX && a.nwork > (a.work ? sms : 4 * sms);
+    a.dynamic = max_ctas <= 0 && a.nwork <= INT32_MAX &&
+                (a.work ? a.nwork > sms : a.nwork > 4 * sms && a.mode != MIXER_VIS_STORE_I32);
     if (a.dynamic) return a.nwork;
     const int64_t grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
     return a.nwork < grid ? a.nwork : grid;
