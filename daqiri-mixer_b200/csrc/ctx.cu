@@ -289,7 +289,9 @@ extern "C" int mixer_reset(mixer_ctx* c, void* stream) {
 
 // Corner-turn + GEMM over nheaps heaps: host packets in chunks of max_heaps (the
 // staging buffers; the copy over PCIe hides the launches), device packets in
-// equal chunks of at most the planes' length.
+// equal chunks of at most the planes' length where that is more than max_heaps.
+// Chunks of max_heaps are never made equal: one of 131 072 heaps is a burst the
+// corner-turn takes, one of 65 537 (odd) is not.
 static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uint32_t seq0,
                           int32_t on_device, void* stream, int32_t mode, void* vis) {
     if (!c || !packets || nheaps <= 0) return MIXER_EINVAL;
@@ -301,7 +303,7 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
     const int64_t most =
         on_device ? std::max<int64_t>(c->kt_planes / d.tpkt, d.max_heaps) : d.max_heaps;
     const int64_t chunks = (nheaps + most - 1) / most;
-    const int64_t step = on_device ? (nheaps + chunks - 1) / chunks : most;
+    const int64_t step = most > d.max_heaps ? (nheaps + chunks - 1) / chunks : most;
     const int64_t kt = step > d.max_heaps ? (step * d.tpkt + 127) / 128 * 128 : c->kt_max;
     for (int64_t h0 = 0; h0 < nheaps; h0 += step) {
         const int32_t nh = (int32_t)((nheaps - h0) < step ? (nheaps - h0) : step);

@@ -857,3 +857,26 @@ def test_context_gives_long_planes_back(cuda):
         assert np.array_equal(dump, (2 * ref).astype(np.float32))
         del fill
     torch.cuda.empty_cache()
+
+
+# ------------------------------------- context chunks that the corner-turn accepts
+
+def test_context_chunks_of_max_heaps(cuda):
+    """One heap more than a long max_heaps: chunks of 131 072 and 1, not two of 65 537."""
+    import torch
+    nant, nch, tpkt, max_heaps = 1, 1, 16, 131072
+    nheaps, stride = max_heaps + 1, 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(11)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    mixer.restamp_seq(pk, nheaps * nant, stride, 3)
+    _sync()
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=1, grid=16,
+                            pkt_stride=stride, max_heaps=max_heaps) as ctx:
+        ctx.correlate(pk, nheaps, 3)
+        out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+        ctx.read_vis_i64(out)
+        _sync()
+        assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
+        st = ctx.stats()
+        assert st["samples"] == nheaps * tpkt and st["seq_errors"] == 0 and st["kernel_err"] == 0
