@@ -33,9 +33,10 @@ struct mixer_ctx {
     int64_t vis_elems;
     int64_t* vis64;
     int32_t* vis32;
-    int8_t* planes;
-    int64_t kt_max;      // samples of max_heaps heaps
-    int64_t kt_planes;   // samples the planes hold (at least kt_max)
+    int8_t* planes;        // one address for the context's life: graphs keep it
+    int64_t kt_max;        // samples the planes hold: max_heaps heaps
+    int8_t* long_planes;   // may be given back: for launches outside capture only
+    int64_t kt_long;       // samples the long planes hold (0: none)
     uint8_t* stage[2];
     size_t stage_bytes;
     cudaEvent_t stage_free[2];
@@ -116,6 +117,7 @@ extern "C" int mixer_destroy(mixer_ctx* c) {
     cudaFree(c->vis64);
     cudaFree(c->vis32);
     cudaFree(c->planes);
+    cudaFree(c->long_planes);
     for (int s = 0; s < 2; ++s) {
         cudaFree(c->stage[s]);
         if (c->stage_free[s]) cudaEventDestroy(c->stage_free[s]);
@@ -142,41 +144,53 @@ extern "C" int mixer_destroy(mixer_ctx* c) {
 // 4096); 1024 elements x 256 channels, 256 heaps 9.50 -> 4.32 ms; 60 x 64, 300
 // heaps in chunks of 8 615 -> 116 us.  Past 1 GiB of planes the shorter length
 // costs nothing (1024 x 256: 4.32 against 4.33 ms).  At most a sixteenth of
-// the device's free memory goes into it; otherwise, or when the allocation
-// fails, the planes hold max_heaps.
+// the device's free memory goes into them; otherwise, or when the allocation
+// fails, such calls run in chunks of max_heaps.
 constexpr int64_t kPlaneSamples = 16384, kPlaneSamplesBig = 8192;
 constexpr int64_t kPlaneBytes = 1LL << 30;
 
-static bool alloc_long_planes(mixer_ctx* c) {
+static void alloc_long_planes(mixer_ctx* c) {
     const int64_t rows = 2LL * c->d.nch * c->d.nant;
     const int64_t kt = rows * kPlaneSamples <= kPlaneBytes ? kPlaneSamples : kPlaneSamplesBig;
     size_t free_b = 0, total_b = 0;
     if (c->kt_max >= kt || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
         (size_t)(rows * kt) > free_b / 16 ||
-        cudaMalloc(&c->planes, (size_t)(rows * kt)) != cudaSuccess) {
+        cudaMalloc(&c->long_planes, (size_t)(rows * kt)) != cudaSuccess) {
         cudaGetLastError();
-        c->planes = nullptr;
-        return false;
+        c->long_planes = nullptr;
+        return;
     }
-    c->kt_planes = kt;
-    return true;
+    c->kt_long = kt;
 }
 
-// Device memory for a buffer made on first use.  When there is none left, planes
-// longer than max_heaps are given back for it.
-static int alloc_late(mixer_ctx* c, void** p, size_t bytes) {
+// Work submitted to the stream goes into a graph.  A graph keeps the addresses
+// of its launches for as long as its owner likes, so it must not hold a buffer
+// that the context may give back.
+static bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
+// Device memory for a buffer made on first use.  When there is none left, the
+// long planes are given back for it.
+static int alloc_late(mixer_ctx* c, void** p, size_t bytes, cudaStream_t st) {
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && c->kt_planes > c->kt_max) {
+    if (e == cudaErrorMemoryAllocation && c->long_planes && !capturing(st)) {
         cudaGetLastError();
         MIXER_CK(cudaDeviceSynchronize());   // launches may still be reading them
-        cudaFree(c->planes);
-        c->planes = nullptr;
-        c->kt_planes = 0;
-        MIXER_CK(cudaMalloc(&c->planes, (size_t)2 * c->d.nch * c->d.nant * c->kt_max));
-        c->kt_planes = c->kt_max;
+        cudaFree(c->long_planes);
+        c->long_planes = nullptr;
+        c->kt_long = 0;
         e = cudaMalloc(p, bytes);
     }
-    if (e != cudaSuccess) *p = nullptr;
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
     MIXER_CK(e);
     return MIXER_OK;
 }
@@ -205,10 +219,8 @@ extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     c->kt_max = (c->kt_max + 15) / 16 * 16;
     CK_OR_FREE(cudaMalloc(&c->vis64, (size_t)c->vis_elems * sizeof(int64_t)));
     CK_OR_FREE(cudaMemset(c->vis64, 0, (size_t)c->vis_elems * sizeof(int64_t)));
-    if (!alloc_long_planes(c)) {
-        c->kt_planes = c->kt_max;
-        CK_OR_FREE(cudaMalloc(&c->planes, (size_t)2 * d->nch * d->nant * c->kt_max));
-    }
+    CK_OR_FREE(cudaMalloc(&c->planes, (size_t)2 * d->nch * d->nant * c->kt_max));
+    alloc_long_planes(c);
     const int G = c->d.grid;
     CK_OR_FREE(cudaMalloc(&c->grid, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
     CK_OR_FREE(cudaMalloc(&c->grid_prev, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
@@ -287,24 +299,26 @@ extern "C" int mixer_reset(mixer_ctx* c, void* stream) {
     return MIXER_OK;
 }
 
-// Corner-turn + GEMM over nheaps heaps: host packets in chunks of max_heaps (the
-// staging buffers; the copy over PCIe hides the launches), device packets in
-// equal chunks of at most the planes' length where that is more than max_heaps.
-// Chunks of max_heaps are never made equal: one of 131 072 heaps is a burst the
-// corner-turn takes, one of 65 537 (odd) is not.
+// Corner-turn + GEMM over nheaps heaps in chunks of max_heaps (from host memory
+// the copy over PCIe hides the launches), or, for longer calls from device memory
+// outside capture, in equal chunks of at most the long planes' length.  Chunks of
+// max_heaps are never made equal: one of 131 072 heaps is a burst the corner-turn
+// takes, one of 65 537 (odd) is not.
 static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uint32_t seq0,
                           int32_t on_device, void* stream, int32_t mode, void* vis) {
     if (!c || !packets || nheaps <= 0) return MIXER_EINVAL;
     const mixer_array_desc& d = c->d;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!c->planes) return MIXER_ENOMEM;   // given back, and no room for short ones either
     const uint8_t* src = static_cast<const uint8_t*>(packets);
     const int64_t heap_bytes = (int64_t)d.nant * d.pkt_stride;
-    const int64_t most =
-        on_device ? std::max<int64_t>(c->kt_planes / d.tpkt, d.max_heaps) : d.max_heaps;
-    const int64_t chunks = (nheaps + most - 1) / most;
-    const int64_t step = most > d.max_heaps ? (nheaps + chunks - 1) / chunks : most;
-    const int64_t kt = step > d.max_heaps ? (step * d.tpkt + 127) / 128 * 128 : c->kt_max;
+    int8_t* planes = c->planes;
+    int64_t kt = c->kt_max, step = d.max_heaps;
+    if (on_device && nheaps > d.max_heaps && c->long_planes && !capturing(st)) {
+        const int64_t most = c->kt_long / d.tpkt, chunks = (nheaps + most - 1) / most;
+        planes = c->long_planes;
+        step = (nheaps + chunks - 1) / chunks;
+        kt = (step * d.tpkt + 127) / 128 * 128;
+    }
     for (int64_t h0 = 0; h0 < nheaps; h0 += step) {
         const int32_t nh = (int32_t)((nheaps - h0) < step ? (nheaps - h0) : step);
         const uint8_t* chunk = src + h0 * heap_bytes;
@@ -312,7 +326,8 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
         if (!on_device) {
             const int s = c->cur;
             if (!c->stage[s]) {
-                const int rc = alloc_late(c, reinterpret_cast<void**>(&c->stage[s]), c->stage_bytes);
+                const int rc = alloc_late(c, reinterpret_cast<void**>(&c->stage[s]), c->stage_bytes,
+                                          st);
                 if (rc != MIXER_OK) return rc;
             }
             if (c->stage_used[s]) MIXER_CK(cudaStreamWaitEvent(c->copy_stream, c->stage_free[s], 0));
@@ -324,9 +339,9 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
         }
         const uint32_t sq = seq0 + (uint32_t)(h0 * d.nant);
         int rc = mixer_corner_turn(dev_chunk, d.pkt_stride, d.hdr_bytes, d.nant, d.nch, d.tpkt, nh,
-                                   sq, c->planes, kt, 0, c->d_seq_err, c->d_err, stream);
+                                   sq, planes, kt, 0, c->d_seq_err, c->d_err, stream);
         if (rc != MIXER_OK) return rc;
-        rc = mixer_xcorr_tri(c->planes, d.nant, d.nch, kt, 0, (int64_t)nh * d.tpkt, mode, vis,
+        rc = mixer_xcorr_tri(planes, d.nant, d.nch, kt, 0, (int64_t)nh * d.tpkt, mode, vis,
                              c->d_err, stream);
         if (rc != MIXER_OK) return rc;
         if (!on_device) {
@@ -352,7 +367,8 @@ extern "C" int mixer_correlate_i32(mixer_ctx* c, const void* packets, int64_t nh
     if (c->i32_samples + nheaps * c->d.tpkt > MIXER_KMAX_I32) return MIXER_EOVERFLOW;
     if (!c->vis32) {
         const int rc = alloc_late(c, reinterpret_cast<void**>(&c->vis32),
-                                  (size_t)c->vis_elems * sizeof(int32_t));
+                                  (size_t)c->vis_elems * sizeof(int32_t),
+                                  static_cast<cudaStream_t>(stream));
         if (rc != MIXER_OK) return rc;
         MIXER_CK(cudaMemsetAsync(c->vis32, 0, (size_t)c->vis_elems * sizeof(int32_t),
                                  static_cast<cudaStream_t>(stream)));
@@ -379,7 +395,8 @@ extern "C" int mixer_dump(mixer_ctx* c, float* out, int32_t out_on_device, void*
     const size_t n = (size_t)c->d.nch * 2 * c->d.nant * c->d.nant;
     if (out_on_device) return mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, out, stream);
     int rc = c->dump_dev ? MIXER_OK
-                         : alloc_late(c, reinterpret_cast<void**>(&c->dump_dev), n * sizeof(float));
+                         : alloc_late(c, reinterpret_cast<void**>(&c->dump_dev), n * sizeof(float),
+                                      static_cast<cudaStream_t>(stream));
     if (rc != MIXER_OK) return rc;
     rc = mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, c->dump_dev, stream);
     if (rc != MIXER_OK) return rc;
@@ -424,7 +441,7 @@ extern "C" int mixer_read_vis_i64(mixer_ctx* c, int64_t* out, int32_t full_squar
     if (out_on_device) return mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, out, stream);
     int rc = c->unpack_dev
                  ? MIXER_OK
-                 : alloc_late(c, reinterpret_cast<void**>(&c->unpack_dev), n * sizeof(int64_t));
+                 : alloc_late(c, reinterpret_cast<void**>(&c->unpack_dev), n * sizeof(int64_t), st);
     if (rc != MIXER_OK) return rc;
     rc = mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, c->unpack_dev, stream);
     if (rc != MIXER_OK) return rc;

@@ -280,10 +280,10 @@ typedef struct mixer_array_desc {
     int32_t pkt_stride;  /* bytes between packets in input buffers            */
     int32_t hdr_bytes;   /* payload offset inside a packet                    */
     int32_t max_heaps;   /* most heaps per antenna given to one correlate call;
-                          * longer calls run in chunks: of max_heaps from host
-                          * memory, of up to 16384 samples from device memory
-                          * where a sixteenth of the free memory holds the
-                          * context's planes of that length                  */
+                          * longer calls run in chunks of max_heaps, or, from
+                          * device memory outside stream capture, of up to 16384
+                          * samples where a sixteenth of the free memory holds
+                          * planes of that length                            */
 } mixer_array_desc;
 
 typedef struct mixer_ctx mixer_ctx;
@@ -301,7 +301,9 @@ int mixer_reset(mixer_ctx* ctx, void* stream);
  * packets, h-major), accumulated straight into the int64 cube.  packets are
  * device memory if packets_on_device, else host memory (pinned for async
  * copies) which is staged through the context.  The gpu_thread body of
- * src/rx_host_corr.cu:159-170 with the flush fused. */
+ * src/rx_host_corr.cu:159-170 with the flush fused.  With device packets the
+ * call may be captured into a CUDA graph: it then works only in buffers that
+ * keep their address until mixer_destroy, in chunks of max_heaps. */
 int mixer_correlate(mixer_ctx* ctx, const void* packets, int64_t nheaps, uint32_t seq0,
                     int32_t packets_on_device, void* stream);
 /* Reference-style split: V32 += X X^H into the context's int32 cube

@@ -880,3 +880,43 @@ def test_context_chunks_of_max_heaps(cuda):
         assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
         st = ctx.stats()
         assert st["samples"] == nheaps * tpkt and st["seq_errors"] == 0 and st["kernel_err"] == 0
+
+
+# ----------------------------- a captured call, after the context gave memory back
+
+def test_captured_correlate_outlives_long_planes(cuda):
+    """Replays of a captured call write only to buffers the context still owns."""
+    import torch
+    nant, nch, tpkt, nheaps = 1000, 20, 16, 5
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(4)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    torch.cuda.empty_cache()
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=32, grid=64,
+                            pkt_stride=stride, max_heaps=2) as ctx:
+        ctx.correlate(pk, nheaps)                   # through the long planes
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            ctx.correlate(pk, nheaps)
+        g.replay()
+        _sync()
+        # leave 100 MB: the 160 MB dump makes the context give its 655 MB back
+        fill = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (100 << 20)), dtype=torch.uint8,
+                           device=cuda)
+        dump = np.zeros(ref.shape, dtype=np.float32)
+        ctx.dump(dump, on_device=False)
+        _sync()
+        assert np.array_equal(dump, (2 * ref).astype(np.float32))
+        room = torch.cuda.mem_get_info()[0] - (100 << 20)
+        assert room > 300 << 20                     # where the long planes were
+        other = torch.full((room,), 7, dtype=torch.uint8, device=cuda)
+        g.replay()
+        ctx.correlate(pk, nheaps)                   # in chunks of max_heaps
+        ctx.dump(dump, on_device=False)
+        _sync()
+        assert np.array_equal(dump, (4 * ref).astype(np.float32))
+        assert int(other.min()) == 7 and int(other.max()) == 7
+        assert ctx.stats()["kernel_err"] == 0
+        del fill, other, g
+    torch.cuda.empty_cache()
