@@ -37,6 +37,7 @@ struct mixer_ctx {
     int64_t kt_max;        // samples the planes hold: max_heaps heaps
     int8_t* long_planes;   // may be given back: for launches outside capture only
     int64_t kt_long;       // samples the long planes hold (0: none)
+    bool long_tried;       // they are asked for once
     uint8_t* stage[2];
     size_t stage_bytes;
     cudaEvent_t stage_free[2];
@@ -51,6 +52,7 @@ struct mixer_ctx {
     float* vmin;
     float* dump_dev;
     int64_t* unpack_dev;
+    int32_t dump_nch, unpack_nch;   // channels these hold
     uint32_t* d_seq_err;
     int32_t* d_err;
     int64_t samples;
@@ -143,24 +145,31 @@ extern "C" int mixer_destroy(mixer_ctx* c) {
 // array, 512 heaps and dump 1368 -> 751 us (787 with 8192 samples, 870 with
 // 4096); 1024 elements x 256 channels, 256 heaps 9.50 -> 4.32 ms; 60 x 64, 300
 // heaps in chunks of 8 615 -> 116 us.  Past 1 GiB of planes the shorter length
-// costs nothing (1024 x 256: 4.32 against 4.33 ms).  At most a sixteenth of
-// the device's free memory goes into them; otherwise, or when the allocation
-// fails, such calls run in chunks of max_heaps.
+// costs nothing (1024 x 256: 4.32 against 4.33 ms).  Allocated by the first call
+// that uses them, so that a context fed from host memory or max_heaps at a time
+// holds none.  At most a sixteenth of the device's free memory goes into them;
+// otherwise, or when the allocation fails, such calls run in chunks of max_heaps.
 constexpr int64_t kPlaneSamples = 16384, kPlaneSamplesBig = 8192;
 constexpr int64_t kPlaneBytes = 1LL << 30;
 
 static void alloc_long_planes(mixer_ctx* c) {
+    c->long_tried = true;
     const int64_t rows = 2LL * c->d.nch * c->d.nant;
     const int64_t kt = rows * kPlaneSamples <= kPlaneBytes ? kPlaneSamples : kPlaneSamplesBig;
+    if (c->kt_max >= kt) return;
+    // A call with device packets may run beside another thread's capture, which
+    // an allocation in the default mode would invalidate.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     size_t free_b = 0, total_b = 0;
-    if (c->kt_max >= kt || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
-        (size_t)(rows * kt) > free_b / 16 ||
-        cudaMalloc(&c->long_planes, (size_t)(rows * kt)) != cudaSuccess) {
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && (size_t)(rows * kt) <= free_b / 16 &&
+        cudaMalloc(&c->long_planes, (size_t)(rows * kt)) == cudaSuccess) {
+        c->kt_long = kt;
+    } else {
         cudaGetLastError();
         c->long_planes = nullptr;
-        return;
     }
-    c->kt_long = kt;
+    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 // Work submitted to the stream goes into a graph.  A graph keeps the addresses
@@ -220,7 +229,6 @@ extern "C" int mixer_create(const mixer_array_desc* d, mixer_ctx** out) {
     CK_OR_FREE(cudaMalloc(&c->vis64, (size_t)c->vis_elems * sizeof(int64_t)));
     CK_OR_FREE(cudaMemset(c->vis64, 0, (size_t)c->vis_elems * sizeof(int64_t)));
     CK_OR_FREE(cudaMalloc(&c->planes, (size_t)2 * d->nch * d->nant * c->kt_max));
-    alloc_long_planes(c);
     const int G = c->d.grid;
     CK_OR_FREE(cudaMalloc(&c->grid, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
     CK_OR_FREE(cudaMalloc(&c->grid_prev, (size_t)d->nch * G * G * 2 * sizeof(int64_t)));
@@ -313,7 +321,9 @@ static int correlate_impl(mixer_ctx* c, const void* packets, int64_t nheaps, uin
     const int64_t heap_bytes = (int64_t)d.nant * d.pkt_stride;
     int8_t* planes = c->planes;
     int64_t kt = c->kt_max, step = d.max_heaps;
-    if (on_device && nheaps > d.max_heaps && c->long_planes && !capturing(st)) {
+    const bool longer = on_device && nheaps > d.max_heaps && !capturing(st);
+    if (longer && !c->long_tried) alloc_long_planes(c);
+    if (longer && c->long_planes) {
         const int64_t most = c->kt_long / d.tpkt, chunks = (nheaps + most - 1) / most;
         planes = c->long_planes;
         step = (nheaps + chunks - 1) / chunks;
@@ -390,19 +400,32 @@ extern "C" int mixer_integrate(mixer_ctx* c, void* stream) {
     return rc;
 }
 
+// A full square to host memory through a device buffer made on first use, of all
+// the channels or of as many as there is room for.
+template <typename T, typename F>
+static int square_to_host(mixer_ctx* c, T*& buf, int32_t& held, T* out, F unpack, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t plane = (size_t)2 * c->d.nant * c->d.nant;   // elements of one channel
+    for (int32_t n = c->d.nch; !buf; n = (n + 1) / 2) {
+        const int rc = alloc_late(c, reinterpret_cast<void**>(&buf), n * plane * sizeof(T), st);
+        if (rc != MIXER_OK && (rc != MIXER_ENOMEM || n == 1)) return rc;
+        held = n;
+    }
+    const int64_t cube = c->vis_elems / c->d.nch;
+    for (int32_t c0 = 0; c0 < c->d.nch; c0 += held) {
+        const int32_t n = std::min(held, c->d.nch - c0);
+        const int rc = unpack(c->vis64 + c0 * cube, c->d.nant, n, buf, stream);
+        if (rc != MIXER_OK) return rc;
+        MIXER_CK(cudaMemcpyAsync(out + c0 * plane, buf, n * plane * sizeof(T), cudaMemcpyDeviceToHost,
+                                 st));
+    }
+    return MIXER_OK;
+}
+
 extern "C" int mixer_dump(mixer_ctx* c, float* out, int32_t out_on_device, void* stream) {
     if (!c || !out) return MIXER_EINVAL;
-    const size_t n = (size_t)c->d.nch * 2 * c->d.nant * c->d.nant;
     if (out_on_device) return mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, out, stream);
-    int rc = c->dump_dev ? MIXER_OK
-                         : alloc_late(c, reinterpret_cast<void**>(&c->dump_dev), n * sizeof(float),
-                                      static_cast<cudaStream_t>(stream));
-    if (rc != MIXER_OK) return rc;
-    rc = mixer_vis_dump_f32(c->vis64, c->d.nant, c->d.nch, c->dump_dev, stream);
-    if (rc != MIXER_OK) return rc;
-    MIXER_CK(cudaMemcpyAsync(out, c->dump_dev, n * sizeof(float), cudaMemcpyDeviceToHost,
-                             static_cast<cudaStream_t>(stream)));
-    return MIXER_OK;
+    return square_to_host(c, c->dump_dev, c->dump_nch, out, mixer_vis_dump_f32, stream);
 }
 
 extern "C" int mixer_dump_to_file(mixer_ctx* c, const char* path, void* stream) {
@@ -437,16 +460,8 @@ extern "C" int mixer_read_vis_i64(mixer_ctx* c, int64_t* out, int32_t full_squar
                                  out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st));
         return MIXER_OK;
     }
-    const size_t n = (size_t)c->d.nch * 2 * c->d.nant * c->d.nant;
     if (out_on_device) return mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, out, stream);
-    int rc = c->unpack_dev
-                 ? MIXER_OK
-                 : alloc_late(c, reinterpret_cast<void**>(&c->unpack_dev), n * sizeof(int64_t), st);
-    if (rc != MIXER_OK) return rc;
-    rc = mixer_vis_unpack_i64(c->vis64, c->d.nant, c->d.nch, c->unpack_dev, stream);
-    if (rc != MIXER_OK) return rc;
-    MIXER_CK(cudaMemcpyAsync(out, c->unpack_dev, n * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    return MIXER_OK;
+    return square_to_host(c, c->unpack_dev, c->unpack_nch, out, mixer_vis_unpack_i64, stream);
 }
 
 extern "C" int mixer_image(mixer_ctx* c, float* img, float* vmax, float* vmin, int32_t delta,

@@ -283,7 +283,8 @@ typedef struct mixer_array_desc {
                           * longer calls run in chunks of max_heaps, or, from
                           * device memory outside stream capture, of up to 16384
                           * samples where a sixteenth of the free memory holds
-                          * planes of that length                            */
+                          * planes of that length, which the first such call
+                          * allocates                                        */
 } mixer_array_desc;
 
 typedef struct mixer_ctx mixer_ctx;

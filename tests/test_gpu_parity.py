@@ -920,3 +920,151 @@ def test_captured_correlate_outlives_long_planes(cuda):
         assert ctx.stats()["kernel_err"] == 0
         del fill, other, g
     torch.cuda.empty_cache()
+
+
+# ------------------------------------------- when a context holds the long planes
+
+def _held(fn):
+    """Device memory that a call leaves allocated."""
+    import torch
+    _sync()
+    before = torch.cuda.mem_get_info()[0]
+    fn()
+    _sync()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("i32", [False, True])
+def test_context_long_planes_on_first_use(cuda, i32):
+    """Calls that do not use them leave no long planes behind; three uneven long chunks."""
+    import torch
+    nant, nch, tpkt, nheaps, short = 96, 24, 16, 2501, 3     # 75 MB for 1024 heaps
+    stride, long_bytes = 64 + 2 * nch * tpkt, 2 * nch * nant * 16384
+    rng = np.random.default_rng(nant)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    mixer.restamp_seq(pk, nheaps * nant, stride, 9)
+    _sync()
+    host = pk.cpu()
+
+    def ref(n):
+        return oracle.correlate(oracle.corner_turn(host[:n * nant * stride].numpy(), nant, nch, tpkt, n))
+
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=12, grid=32,
+                            pkt_stride=stride, max_heaps=short) as ctx:
+        call = ctx.correlate_i32 if i32 else ctx.correlate
+        out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+        call(pk, 1, 9)                                       # makes the int32 cube
+        quiet = [_held(lambda: call(pk, short, 9)),
+                 _held(lambda: call(host.pin_memory(), 2 * short, 9, on_device=False))]
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            call(pk, 2 * short, 9)
+        quiet.append(_held(g.replay))
+        assert max(quiet) < long_bytes // 2, quiet
+        ctx.reset()
+        assert long_bytes <= _held(lambda: call(pk, nheaps, 9)) < long_bytes + (16 << 20)
+        assert _held(lambda: call(pk, 1500, 9)) < long_bytes // 2
+        ctx.integrate()
+        ctx.read_vis_i64(out)
+        _sync()
+        expect = ref(nheaps) + ref(1500)
+        assert np.array_equal(out.cpu().numpy().reshape(expect.shape), expect)
+        assert ctx.stats()["seq_errors"] == 0 and ctx.stats()["kernel_err"] == 0
+        del g
+
+
+def test_context_planes_longer_than_the_long_ones(cuda):
+    """max_heaps past 16 384 samples: no second planes."""
+    import torch
+    nant, nch, tpkt, max_heaps, nheaps = 64, 16, 16, 1025, 2100
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(nant)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=8, grid=16,
+                            pkt_stride=stride, max_heaps=max_heaps) as ctx:
+        out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+        ctx.correlate(pk, 1)
+        ctx.reset()
+        assert _held(lambda: ctx.correlate(pk, nheaps)) < 16 << 20
+        ctx.read_vis_i64(out)
+        _sync()
+        assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
+
+
+def test_context_of_host_packets_holds_no_long_planes(cuda):
+    import torch
+    nant, nch, tpkt, nheaps = 300, 40, 16, 2
+    stride = 64 + 2 * nch * tpkt
+    kw = dict(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=20, grid=64, pkt_stride=stride,
+              max_heaps=nheaps)
+    pk = torch.zeros(nheaps * nant * stride, dtype=torch.uint8).pin_memory()
+    first = mixer.ArrayContext(**kw)
+    more = []
+    try:
+        each = _held(lambda: more.append(mixer.ArrayContext(**kw)))
+        # cube, planes, grids and image (in blocks of 2 MB), without long planes (393 MB)
+        own = mixer.vis_elems(nant, nch) * 8 + 2 * nch * nant * nheaps * tpkt + nch * 64 * 64 * 36
+        assert own - (8 << 20) <= each < own + (64 << 20)
+        assert _held(lambda: first.correlate(pk, 1, on_device=False)) < 64 << 20
+    finally:
+        for ctx in [first] + more:
+            ctx.close()
+
+
+@pytest.mark.parametrize("read", ["dump", "read_vis_i64"])
+def test_context_host_output_in_pieces(cuda, read):
+    """A full square whose device buffer does not fit comes out through a smaller one."""
+    import torch
+    nant, nch, tpkt, nheaps = 700, 41, 16, 2
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(8)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    torch.cuda.empty_cache()
+    with mixer.ArrayContext(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=30, grid=64,
+                            pkt_stride=stride, max_heaps=nheaps) as ctx:
+        ctx.correlate(pk, nheaps)
+        warm = torch.empty(nch * 2 * nant * nant, dtype=torch.float32, device=cuda)
+        ctx.dump(warm)
+        del warm
+        torch.cuda.empty_cache()
+        _sync()
+        # leave 100 MB: less than the square of all 41 channels (161 MB, 321 MB in int64)
+        fill = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (100 << 20)), dtype=torch.uint8,
+                           device=cuda)
+        out = np.zeros(ref.shape, dtype=np.float32 if read == "dump" else np.int64)
+        for times in (1, 2):                        # the second through the buffer of the first
+            getattr(ctx, read)(out, on_device=False)
+            _sync()
+            assert np.array_equal(out, (times * ref).astype(out.dtype))
+            ctx.correlate(pk, nheaps)
+        del fill
+    torch.cuda.empty_cache()
+
+
+def test_context_long_call_beside_a_capture(cuda):
+    """The first long call allocates without ending a capture on another stream."""
+    import torch
+    nant, nch, tpkt, nheaps = 24, 4, 16, 40
+    stride = 64 + 2 * nch * tpkt
+    rng = np.random.default_rng(6)
+    pk = torch.from_numpy(rng.integers(0, 256, size=nheaps * nant * stride, dtype=np.uint8)).to(cuda)
+    ref = oracle.correlate(oracle.corner_turn(pk.cpu().numpy(), nant, nch, tpkt, nheaps))
+    kw = dict(nant=nant, nch=nch, tpkt=tpkt, ksub=tpkt, side_x=6, grid=16, pkt_stride=stride,
+              max_heaps=8)
+    with mixer.ArrayContext(**kw) as ctx, mixer.ArrayContext(**kw) as recorded:
+        side = torch.cuda.Stream()
+        _sync()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            recorded.correlate(pk, nheaps)
+            ctx.correlate(pk, nheaps, stream=side)
+        g.replay()
+        _sync()
+        for c in (ctx, recorded):
+            out = torch.empty(nch * 2 * nant * nant, dtype=torch.int64, device=cuda)
+            c.read_vis_i64(out)
+            _sync()
+            assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
+        del g
