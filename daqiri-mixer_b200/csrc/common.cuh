@@ -36,7 +36,10 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // ---- dependent launches -----------------------------------------------------
 // A kernel launched by launch_dependent may start before the kernel ahead of
 // it on the stream has finished; nothing it reads or writes in global memory
-// may be touched before pdl_wait.  pdl_trigger lets the next such kernel start
+// may be touched before pdl_wait.  Nor may its pointers be declared
+// __restrict__: what the kernel ahead still writes is not constant for this
+// one's life, as read-only loads require, and the compiler could move such
+// loads over the wait.  pdl_trigger lets the next such kernel start
 // once every CTA has called it (or exited).  What it saves is the launch and
 // the set-up between two kernels: 64 elements x 16 channels, K 256 (corner-turn
 // and GEMM) 12.3 -> 10.9 us; 256 x 128, K 1024 78.2 -> 73.4; 200 x 128, K 1536

@@ -21,9 +21,9 @@ namespace mixer {
 namespace {
 
 __global__ void __launch_bounds__(256)
-    k_corner_turn(const uint8_t* __restrict__ pk, int64_t pkt_stride, int hdr, int nant, int nch,
+    k_corner_turn(const uint8_t* pk, int64_t pkt_stride, int hdr, int nant, int nch,
                   int tpkt, int nheaps, int hg, int nchg, uint32_t seq0,
-                  int8_t* __restrict__ planes, int64_t kt, int64_t k0, uint32_t* seq_err,
+                  int8_t* planes, int64_t kt, int64_t k0, uint32_t* seq_err,
                   int32_t* err) {
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ __align__(8) uint64_t bar_store;

@@ -67,8 +67,8 @@ __device__ __forceinline__ int pmod(int v, int g) {
 // measured 473 us there.
 template <int kThreads, int kUnroll, bool kWhole>
 __global__ void __launch_bounds__(kThreads)
-    k_grid_tiles(const long long* __restrict__ vis, int nant, int ntiles, int sx, int G,
-                 unsigned long long* __restrict__ grid, longlong2* __restrict__ prev) {
+    k_grid_tiles(const long long* vis, int nant, int ntiles, int sx, int G,
+                 unsigned long long* grid, longlong2* prev) {
     extern __shared__ unsigned long long win[];
     __shared__ unsigned long long diag[2];
     constexpr int kGroups = kThreads / 128;
@@ -211,8 +211,7 @@ __global__ void k_grid_delta(long long* __restrict__ grid, long long* __restrict
 }
 
 __global__ void __launch_bounds__(512)
-    k_image_fft(const long long* __restrict__ grid, int G, int logG, float* __restrict__ img,
-                float* __restrict__ vmax, float* __restrict__ vmin) {
+    k_image_fft(const long long* grid, int G, int logG, float* img, float* vmax, float* vmin) {
     extern __shared__ float2 S[];               // [G][G] then twiddles [G/2]
     float2* tw = S + G * G;
     __shared__ float red_max[16], red_min[16];
@@ -326,8 +325,7 @@ __device__ __forceinline__ void warp_fft(float2 (&v)[G / 32], const float2* __re
 
 template <int G>
 __global__ void __launch_bounds__(1024)
-    k_image_fft_warp(const long long* __restrict__ grid, float* __restrict__ img,
-                     float* __restrict__ vmax, float* __restrict__ vmin) {
+    k_image_fft_warp(const long long* grid, float* img, float* vmax, float* vmin) {
     constexpr int E = G / 32, H = G / 2, P = G + 1, LOGG = G == 32 ? 5 : (G == 64 ? 6 : 7);
     extern __shared__ float2 S[];                      // [G][G + 1] then twiddles [G / 2]
     float2* tw = S + G * P;

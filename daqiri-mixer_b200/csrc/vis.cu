@@ -15,7 +15,7 @@ namespace mixer {
 namespace {
 
 __global__ void __launch_bounds__(256)
-    k_vis_flush(int4* __restrict__ v32, longlong2* __restrict__ v64, int64_t n4) {
+    k_vis_flush(int4* v32, longlong2* v64, int64_t n4) {
     pdl_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -59,7 +59,7 @@ __device__ __forceinline__ long long conv<long long>(long long v) {
 // (row stride 129: conflict-free both ways).
 template <typename T>
 __global__ void __launch_bounds__(256)
-    k_vis_unpack(const long long* __restrict__ vis, int nant, int ntiles, T* __restrict__ out) {
+    k_vis_unpack(const long long* vis, int nant, int ntiles, T* out) {
     __shared__ T s[32][129];
     const int ng = blockIdx.x;
     const int t = blockIdx.y >> 1, p = blockIdx.y & 1;
