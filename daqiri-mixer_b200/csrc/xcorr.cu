@@ -225,6 +225,12 @@ __device__ __forceinline__ Item get_item(const XcorrArgs& a, const CUtensorMap* 
     return it;
 }
 
+// Chunks of item w (of a K range, at most).
+__device__ __forceinline__ int item_chunks(const XcorrArgs& a, int64_t w) {
+    if (a.work) return (int)a.work[w].nkc;
+    return w < a.nwhole ? a.nkc : a.kpart;
+}
+
 // Four 32x32b.x16 TMEM loads (16 columns each) and the wait, in one asm
 // statement so no use of the results can be scheduled before the wait.
 __device__ __forceinline__ void tmem_ld4_x16(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -344,17 +350,20 @@ __device__ __forceinline__ void red_add(int* p, int32_t x) {
 // 3072 685 -> 607, K 8192 1553 -> 1441; 1024 x 64, K 2048 298 -> 279; 640 x 48,
 // K 8192 257 -> 247; int32, 4096 x 8, K 1024 263 -> 254, K 2048 413 -> 370.
 // Shorter tiles are bound by the cube's traffic itself and are not paced.  The
-// time spread over is a tile's MMA time (1024 clocks a chunk), 1.2 times that
-// for int64 (1.0: 0-7 % slower, 0.9: 3-8 %), at most 64 x kPaceMax clocks.
+// time spread over is the MMA time (1024 clocks a chunk) of the tile or of the
+// next one, whichever is shorter: adds that outlast the next tile's MMAs hold
+// up the tile after it (K ranges behind whole rounds, 128 x 760, K 8192 333 ->
+// 322 us against the tile's own time).  1.2 times that for int64 (1.0: 0-7 %
+// slower, 0.9: 3-8 %), at most 64 x kPaceMax clocks.
 constexpr int kPaceCols = 4;
 constexpr int kPaceChunks64 = 16, kPaceChunks32 = 8;   // shortest tile paced
 constexpr int kPaceMax64 = 600, kPaceMax32 = 400;      // clocks per column
 
 struct Pace {
     uint32_t t0, dt, due;   // start, clocks per step, clocks after t0 at which the next is due
-    __device__ __forceinline__ void begin(const Item& it) {
-        const int col = it.mode == MIXER_VIS_ACC_I64 ? min(it.nkc * 19, kPaceMax64)
-                                                     : min(it.nkc * 16, kPaceMax32);
+    __device__ __forceinline__ void begin(int mode, int nkc) {
+        const int col = mode == MIXER_VIS_ACC_I64 ? min(nkc * 19, kPaceMax64)
+                                                  : min(nkc * 16, kPaceMax32);
         dt = (uint32_t)(col * kPaceCols);
         due = 0;
         t0 = now();
@@ -784,10 +793,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             Pace pace;
             // Not in short launches, nor for the CTA's last tile, which no MMAs follow.
             const bool many = args.dynamic || args.nwork > 4 * (int64_t)gridDim.x;
+            int beside = 0;   // chunks to spread the adds over
             if (many && it.nkc >= pace_min && !it.tail &&
                 __all_sync(0xffffffffu, mbar_test(bar(IFULL + islot), iphase)) &&
-                witems[islot] >= 0) {
-                pace.begin(it);
+                witems[islot] >= 0)
+                beside = min(it.nkc, item_chunks(args, witems[islot]));
+            if (beside >= pace_min) {
+                pace.begin(it.mode, beside);
 #pragma unroll
                 for (int k = 0; k < kEpiChunks; ++k)
                     store16<true>(it, tb + (size_t)n0_of(k) * kTile + m, &re[16 * k], &im[16 * k],

@@ -1068,3 +1068,47 @@ def test_context_long_call_beside_a_capture(cuda):
             _sync()
             assert np.array_equal(out.cpu().numpy().reshape(ref.shape), ref)
         del g
+
+
+# ------------------------- adds beside a next tile that is shorter than their own
+
+@pytest.mark.parametrize("nch,klen", [
+    (760, 2048),      # 20 tiles behind five rounds, in parts too short to be paced beside
+    (760, 7424),      # parts of nine chunks, the last of four
+])
+def test_xcorr_paced_before_parts(cuda, nch, klen):
+    import torch
+    nant = 128
+    g = torch.Generator(device=cuda).manual_seed(nch)
+    planes = torch.randint(-128, 128, (2, nch, nant, klen), dtype=torch.int8, device=cuda, generator=g)
+    n = mixer.vis_elems(nant, nch)
+    err = _zeros(1, torch.int32, cuda)
+    ref = _zeros(n, torch.int32, cuda)
+    mixer.xcorr_tri(planes, nant, nch, klen, 0, klen, mixer.VIS_STORE_I32, ref, err)
+    for mode, dtype in ((mixer.VIS_ACC_I32, torch.int32), (mixer.VIS_ACC_I64, torch.int64)):
+        vis = torch.full((n,), 5, dtype=dtype, device=cuda)
+        mixer.xcorr_tri(planes, nant, nch, klen, 0, klen, mode, vis, err)
+        _sync()
+        assert torch.equal(vis - 5, ref.to(dtype)), mode
+    assert int(err.item()) == 0
+
+
+def test_batch_items_of_falling_length(cuda):
+    import torch
+    g = torch.Generator(device=cuda).manual_seed(2)
+    shapes = [(128, 300, 2176), (128, 300, 2048), (256, 40, 1024), (128, 200, 128)]
+    err = _zeros(1, torch.int32, cuda)
+    probs, refs = [], []
+    for nant, nch, k in shapes:
+        planes = torch.randint(-128, 128, (2, nch, nant, k), dtype=torch.int8, device=cuda, generator=g)
+        refs.append(_zeros(mixer.vis_elems(nant, nch), torch.int32, cuda))
+        mixer.xcorr_tri(planes, nant, nch, k, 0, k, mixer.VIS_STORE_I32, refs[-1], err)
+        probs.append(dict(planes=planes, nant=nant, nch=nch, kt=k, mode=mixer.VIS_ACC_I64,
+                          vis=_zeros(mixer.vis_elems(nant, nch), torch.int64, cuda)))
+    batch = mixer.Batch(probs)
+    for _ in range(3):
+        batch.run()
+    _sync()
+    for prob, ref in zip(probs, refs):
+        assert torch.equal(prob["vis"], 3 * ref.to(torch.int64))
+    assert int(err.item()) == 0
