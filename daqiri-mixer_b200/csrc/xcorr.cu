@@ -105,7 +105,7 @@ constexpr uint32_t kTmemCols = 512;              // D1 (256) + D2 (256)
 constexpr uint32_t kIdesc = idesc_i8(128, 256);
 
 struct XcorrArgs {
-    int32_t nant, nch, nblk, ntiles;
+    int32_t nant, ntiles;   // ntiles: tiles of a channel
     int32_t kbeg, nkc;   // first sample, number of 128-sample chunks
     int32_t mode;
     int32_t dynamic;     // 1: one CTA per item, taken over by the running ones; 0: CTA b
@@ -1277,8 +1277,6 @@ static int set_smem_attr() {
     return MIXER_OK;
 }
 
-int xcorr_sm_count() { return sm_count(); }
-
 // Pair kernel set-up, once per device: its shared-memory attribute and how
 // many clusters of two CTAs can be resident at once (0: pairs unusable).
 static int pair_clusters() {
@@ -1370,8 +1368,7 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
 // 36.1 us instead of 34.8, in two of eight 42.1 instead of 44.8.
 constexpr int kPartChunks = 2, kPartChunksBehind = 6;
 
-static void split_last_round(XcorrArgs& a, int32_t max_ctas) {
-    const int64_t tiles = (int64_t)a.nch * a.ntiles;
+static void split_last_round(XcorrArgs& a, int64_t tiles, int32_t max_ctas) {
     a.nwhole = a.nwork = tiles;
     a.nsplit = 0;
     a.kpart = a.nkc;
@@ -1429,13 +1426,11 @@ static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t
     if (rc != MIXER_OK) return rc;
     XcorrArgs a;
     a.nant = nant;
-    a.nch = nch;
-    a.nblk = (nant + kTile - 1) / kTile;
-    a.ntiles = a.nblk * (a.nblk + 1) / 2;
+    a.ntiles = mixer_vis_tiles(nant);
     a.kbeg = (int32_t)kbeg;
     a.nkc = (int32_t)((klen + kWorkChunk - 1) / kWorkChunk);
     a.mode = mode;
-    split_last_round(a, max_ctas);
+    split_last_round(a, (int64_t)nch * a.ntiles, max_ctas);
     a.vis = vis;
     a.err = err;
     a.tmaps = nullptr;

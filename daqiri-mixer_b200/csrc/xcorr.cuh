@@ -33,6 +33,5 @@ int xcorr_encode_maps(CUtensorMap* maps, const int8_t* planes, int32_t nant, int
 int xcorr_launch_table(const CUtensorMap* d_tmaps, const XcorrProblem* d_probs,
                        const XcorrWork* d_work, int64_t nwork, int32_t* err, bool ragged,
                        cudaStream_t st);
-int xcorr_sm_count();
 
 }  // namespace mixer
