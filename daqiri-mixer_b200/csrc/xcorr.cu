@@ -31,8 +31,8 @@
 //
 // What bounds it: the int8 tensor rate at the clock the 1000 W cap leaves for
 // long K, the cube's read-modify-write in HBM for short K.  One tile's four
-// products fill TMEM, so the next tile waits for the drain alone (1350 clocks,
-// and 350 more of barriers) instead of for the adds: 128 result registers a
+// products fill TMEM, so the next tile waits for the drain alone (850 clocks;
+// 1000 from its last MMA to the next tile's first) instead of for the adds: 128 result registers a
 // thread, which the register split below pays for.  One B200, against adds straight from TMEM: 4096
 // elements x 64 channels, K 2048 with its corner-turn 5.81 -> 5.49 ms; 1024 x
 // 64, K 2048 int64 328 -> 301 us, K 8192 802 -> 782 us; 200 x 128, K 1536
@@ -345,8 +345,8 @@ __device__ __forceinline__ void red_add(int* p, int32_t x) {
 // rate take all that one SM can read from L2 (64 bytes a clock), so operands
 // that come late are not made up for, and while the adds leave in one burst
 // the operand loads get about a third of that: 16 chunks of MMAs took 28 000
-// clocks beside the int64 adds and 19 300 beside int32 stores, against 16 400
-// alone.  One B200, without -> with: int64, 4096 x 8, K 2048 531 -> 488 us, K
+// clocks beside the int64 adds, against 16 400 alone; paced they take 25 600
+// (int32: 18 500).  One B200, without -> with: int64, 4096 x 8, K 2048 531 -> 488 us, K
 // 3072 685 -> 607, K 8192 1553 -> 1441; 1024 x 64, K 2048 298 -> 279; 640 x 48,
 // K 8192 257 -> 247; int32, 4096 x 8, K 1024 263 -> 254, K 2048 413 -> 370.
 // Shorter tiles are bound by the cube's traffic itself and are not paced.  The
@@ -1366,6 +1366,11 @@ static int pair_launch(const CUtensorMap& map, int32_t nant, int32_t nch, int64_
 // four, 9.0 with eight); behind whole rounds, whose adds are still under way,
 // the parts have to be longer: in two parts of four chunks 222 channels take
 // 36.1 us instead of 34.8, in two of eight 42.1 instead of 44.8.
+// The parts serve the launch that has the GPU to itself.  Several small launches
+// side by side on streams of one graph take longer in parts, whole -> split:
+// eight of 64 x 16, K 4096 27 -> 50 us (one after the other 132 -> 60), four of
+// 256 x 16, K 1024 33 -> 49 (60 -> 55).  A CTA limit of as many CTAs as the
+// launch has tiles keeps them whole.
 constexpr int kPartChunks = 2, kPartChunksBehind = 6;
 
 static void split_last_round(XcorrArgs& a, int64_t tiles, int32_t max_ctas) {
@@ -1400,6 +1405,10 @@ static void split_last_round(XcorrArgs& a, int64_t tiles, int32_t max_ctas) {
 // 192 50.1 -> 44.2 us, 640 x 48, K 1024 55 -> 42, 4096 x 8, K 512 142 -> 136, but
 // 1024 x 64, K 256 60.8 -> 64.8.  Table launches hold items of different lengths and are always taken
 // over; a launch with a CTA limit cannot be, since its grid would be the items.
+// A CTA fills its SM's registers either way, so a kernel on another stream
+// starts when the launch runs out of items unless the limit leaves it SMs: a
+// small flush beside 1024 x 64, K 8192 is done after 830 us, with 144 CTAs
+// after 42 (the GEMM 2-5 % slower).
 static int64_t launch_grid(XcorrArgs& a, int32_t max_ctas) {
     const int64_t sms = sm_count();
     a.dynamic = max_ctas <= 0 && a.nwork <= INT32_MAX &&
@@ -1410,7 +1419,7 @@ static int64_t launch_grid(XcorrArgs& a, int32_t max_ctas) {
 }
 
 // Launch over samples [kbeg, kbeg + klen) with klen <= MIXER_KMAX_I32.
-// At most max_ctas persistent CTAs (<= 0: one per SM).
+// At most max_ctas persistent CTAs (<= 0: every SM).
 static int xcorr_launch(const int8_t* planes, int32_t nant, int32_t nch, int64_t kt, int64_t kbeg,
                         int64_t klen, int32_t mode, void* vis, int32_t max_ctas, int32_t* err,
                         cudaStream_t st) {

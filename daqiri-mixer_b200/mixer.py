@@ -198,9 +198,9 @@ _current_raw = None   # () -> handle of torch's current stream, once torch has C
 
 
 def _bind_current_raw(torch):
-    """torch.cuda.current_stream() builds a Stream object, which took 3.2 of a
-    call's 10 us of host time; the raw handle of the current device's current
-    stream takes 0.2 us where this torch has it."""
+    """torch.cuda.current_stream() builds a Stream object, which took 3.1 us of a
+    call's 10 of host time (and is_available() before it 0.7); the raw handle of
+    the current device's current stream takes 0.2 us where this torch has it."""
     global _current_raw
     device = getattr(torch._C, "_cuda_getDevice", None)
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)

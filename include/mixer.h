@@ -110,10 +110,15 @@ int mixer_xcorr_tri(const int8_t* planes, int32_t nant, int32_t nch, int64_t kt,
                     int64_t kbeg, int64_t klen, int32_t mode, void* vis,
                     int32_t* err, void* stream);
 
-/* Same, with at most max_ctas persistent CTAs (<= 0: one per SM; the pair
- * kernel uses max_ctas / 2 clusters, and max_ctas == 1 selects the one-SM
- * kernel).  Leaving SMs free lets an HBM-bound kernel on another stream (the
- * next corner-turn) run beside the tensor-bound GEMM. */
+/* Same, with at most max_ctas CTAs, which are persistent (<= 0: every SM, with
+ * one CTA per SM at a time; the pair kernel uses max_ctas / 2 clusters, and
+ * max_ctas == 1 selects the one-SM kernel).  A CTA takes an SM's registers to
+ * itself: without a limit a kernel on another stream waits until the launch has
+ * no items left, with a few SMs left free (144 CTAs) it runs at once.  A launch
+ * with fewer tiles than SMs is also split over all of them in K, which is the
+ * fastest for one launch at a time; several such launches side by side on their
+ * own streams are faster with max_ctas = nch * mixer_vis_tiles(nant) each,
+ * which keeps the tiles whole. */
 int mixer_xcorr_tri_ex(const int8_t* planes, int32_t nant, int32_t nch, int64_t kt,
                        int64_t kbeg, int64_t klen, int32_t mode, void* vis,
                        int32_t max_ctas, int32_t* err, void* stream);
